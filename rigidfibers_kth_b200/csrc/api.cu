@@ -734,6 +734,11 @@ rf_status rf_solve_system(rf_handle *h) {
     const int nb = 3 * h->N;
     rf::GmresResult res;
     rf_status status = RF_OK;
+    // a product queued after a device-controlled solve stopped returns at once: not a product to time
+    auto drop_skipped = [h] {
+        if (h->gt.on && h->gt.used >= 2) h->gt.used -= 2;
+    };
+    const bool device_control = m <= rf::kArnoldiMax;
     if (prec == RF_PREC_FP64 && h->p.use_direct_solver) {
         // dgesv (coeffs_and_vels.f90:62,158): LU factors of a copy of A (A
         // itself stays available to rf_get_matrix and rf_matvec), then the two
@@ -782,34 +787,41 @@ rf_status rf_solve_system(rf_handle *h) {
     } else if (prec == RF_PREC_FP64) {
         if (h->shards > 1 && !h->comm)
             return rf::fail(h, RF_ERR_INVALID_ARG, "a row-block shard solves with its communicator (rf_create_sharded)");
-        rf::Gmres<double>::Op A = [h](const double *in, double *out) {
+        rf::Gmres<double>::StopOp A_s = [h](const double *in, double *out, const int *stop) {
             h->launches += 2;
             if (h->comm) {
                 // this shard's rows, then the row blocks of every shard
                 cudaError_t e = timed_product(h, 8.0 * h->lda * h->n, [&] {
                     return rf::launch_gemv<double, double, double, double>(h->A64, h->lda, h->n_loc, h->n, in,
                                                                             h->shard_send, nullptr, h->work64,
-                                                                            h->work_elems, h->sm_count, h->stream);
+                                                                            h->work_elems, h->sm_count, h->stream, stop);
                 });
                 return e == cudaSuccess ? rf::shard_allgather(h, out, 3 * h->N, h->shard_send) : e;
             }
             return timed_product(h, 8.0 * h->lda * h->n, [&] {
                 return rf::launch_gemv<double, double, double, double>(h->A64, h->lda, h->n, h->n, in, out, nullptr,
                                                                        h->work64, h->work_elems, h->sm_count,
-                                                                       h->stream);
+                                                                       h->stream, stop);
             });
         };
-        rf::Gmres<double>::Op P = [h, nb, pc_omega](const double *in, double *out) {
+        rf::Gmres<double>::StopOp P_s = [h, nb, pc_omega](const double *in, double *out, const int *stop) {
             return rf::launch_pair_apply<double>(h->M, nb, h->pc_pairs, RF_MLP_PAIRS, h->Pblocks, h->knn, RF_MLP_K, pc_omega, in, out,
-                                                  h->stream);
+                                                  h->stream, stop);
         };
+        rf::Gmres<double>::Op A = [&A_s](const double *in, double *out) { return A_s(in, out, nullptr); };
+        rf::Gmres<double>::Op P = [&P_s](const double *in, double *out) { return P_s(in, out, nullptr); };
         {
             bool pc_on = use_pc;
             double prev = 1.0;  // residual relative to |b| before this trial
             rf::GmresResult part;
             for (int used = 0;;) {
                 const int budget = pc_on ? std::min(maxit - used, pc_trial) : maxit - used;
-                CK(h, h->gm64->solve(A, pc_on ? &P : nullptr, h->b, h->x, false, tol, budget, &part), "GMRES");
+                if (device_control)
+                    CK(h, h->gm64->solve_device(A_s, pc_on ? &P_s : nullptr, h->b, h->x, false, tol, budget, &part,
+                                                drop_skipped, true),
+                       "GMRES");
+                else
+                    CK(h, h->gm64->solve(A, pc_on ? &P : nullptr, h->b, h->x, false, tol, budget, &part), "GMRES");
                 used += part.iterations;
                 res.iterations += part.iterations;
                 res.matvecs += part.matvecs;
@@ -831,16 +843,18 @@ rf_status rf_solve_system(rf_handle *h) {
         h->stats.residual = res.backward_error;
         h->stats.converged = res.info == 0;
     } else if (prec == RF_PREC_FP32) {
-        rf::Gmres<float>::Op A = [h](const float *in, float *out) {
+        rf::Gmres<float>::StopOp A_s = [h](const float *in, float *out, const int *stop) {
             h->launches += 2;
             return timed_product(h, 4.0 * h->lda * h->n, [&] {
-                return fp32_gemv<float, float, float>(h, in, out, nullptr, h->work32);
+                return fp32_gemv<float, float, float>(h, in, out, nullptr, h->work32, stop);
             });
         };
-        rf::Gmres<float>::Op P = [h, nb, pc_omega](const float *in, float *out) {
+        rf::Gmres<float>::StopOp P_s = [h, nb, pc_omega](const float *in, float *out, const int *stop) {
             return rf::launch_pair_apply<float>(h->M, nb, h->pc_pairs, RF_MLP_PAIRS, h->Pblocks, h->knn, RF_MLP_K, pc_omega, in, out,
-                                                 h->stream);
+                                                 h->stream, stop);
         };
+        rf::Gmres<float>::Op A = [&A_s](const float *in, float *out) { return A_s(in, out, nullptr); };
+        rf::Gmres<float>::Op P = [&P_s](const float *in, float *out) { return P_s(in, out, nullptr); };
         CK(h, (rf::launch_convert<float, double>(h->n, h->x, h->x32, st)), "convert");
         CK(h, (rf::launch_convert<float, double>(h->n, h->b, h->r32, st)), "convert");
         h->launches += 2;
@@ -850,7 +864,12 @@ rf_status rf_solve_system(rf_handle *h) {
             rf::GmresResult part;
             for (int used = 0;;) {
                 const int budget = pc_on ? std::min(maxit - used, pc_trial) : maxit - used;
-                CK(h, h->gm32->solve(A, pc_on ? &P : nullptr, h->r32, h->x32, false, tol, budget, &part), "GMRES");
+                if (device_control)
+                    CK(h, h->gm32->solve_device(A_s, pc_on ? &P_s : nullptr, h->r32, h->x32, false, tol, budget, &part,
+                                                drop_skipped, true),
+                       "GMRES");
+                else
+                    CK(h, h->gm32->solve(A, pc_on ? &P : nullptr, h->r32, h->x32, false, tol, budget, &part), "GMRES");
                 used += part.iterations;
                 res.iterations += part.iterations;
                 res.matvecs += part.matvecs;
@@ -909,11 +928,6 @@ rf_status rf_solve_system(rf_handle *h) {
             return rf::launch_pair_apply<float>(h->M, nb, h->pc_pairs, RF_MLP_PAIRS, h->Pblocks, h->knn, RF_MLP_K, pc_omega, in, out,
                                                  h->stream, stop);
         };
-        // a product queued after the inner solve stopped returns at once: not a product to time
-        auto drop_skipped = [h] {
-            if (h->gt.on && h->gt.used >= 2) h->gt.used -= 2;
-        };
-        const bool device_control = m <= rf::kArnoldiMax;
         double *dnorm = h->dscal;
         const rf::RedBuf &rb = h->rb;
         auto norm_of = [&](const double *v, double *hv) -> cudaError_t {
@@ -982,8 +996,8 @@ rf_status rf_solve_system(rf_handle *h) {
             const double itol_k = std::min(0.5, std::pow(need, 1.0 / left));
             const int budget = pc_on ? std::min(maxit, pc_trial) : maxit;
             if (device_control)
-                e = h->gm32->solve_device(Alo_s, pc_on ? &P_s : nullptr, h->r32, h->d32, itol_k, budget, &res,
-                                          drop_skipped);
+                e = h->gm32->solve_device(Alo_s, pc_on ? &P_s : nullptr, h->r32, h->d32, true, itol_k, budget, &res,
+                                          drop_skipped, false);
             else
                 e = h->gm32->solve(Alo, pc_on ? &P : nullptr, h->r32, h->d32, true, itol_k, budget, &res, false);
             if (e != cudaSuccess) break;

@@ -1,21 +1,28 @@
-// arnoldi.cu - Arnoldi steps of the inner GMRES controlled on the device.
+// arnoldi.cu - Arnoldi steps of GMRES controlled on the device.
 //
-// The inner solves of the mixed-precision refinement stop on the Arnoldi
-// estimate alone, so the whole GMRES(m) cycle can run without the host: the
-// Gram-Schmidt coefficients, the Givens update of the Hessenberg column and
-// the stop test happen in the kernels, and every kernel of the next step
+// The Gram-Schmidt coefficients, the Givens update of the Hessenberg column
+// and the stop test happen in the kernels, and every kernel of the next step
 // reads the stop flag first and returns at once when it is set.  The host
 // then queues step j + 1 before it learns (from host-mapped memory) whether
 // step j stopped: the GPU never waits for the host between steps, and a
-// step queued after the stop costs a few empty launches.
+// step queued after the stop costs a few empty launches.  The inner solves of
+// the mixed-precision refinement and the FP64 and FP32 GMRES all run this way
+// (restart lengths up to kArnoldiMax; longer ones use the host-controlled
+// solver).  What bounds a small system is the number of dependent launches: a
+// step is the product's two kernels, three orthogonalisation passes and one
+// scaling, where the host-controlled solver takes j + 5 launches, a copy and
+// a wait of the host.  Whole time steps,
+// FP64: M = 100 (18 iterations) 1.70 -> 0.96 ms, M = 333 (N = 3) 2.24 -> 1.51
+// ms, M = 1000 (products of 0.28 ms) 13.9 -> 12.8 ms; FP32 M = 1000 6.04 ->
+// 5.57 ms.
 //
 // Orthogonalisation: classical Gram-Schmidt applied twice (CGS2), fused into
 // three passes over the basis: (1) h1 = V^T w; (2) w -= V h1, h2 = V^T w;
 // (3) w -= V h2, |w|.  The reference solver (dGMRES.f with icntl(5) = 0) uses
-// modified Gram-Schmidt, one pass per basis vector; the FP64 GMRES of this
-// library keeps that order (its iterates are compared with the oracle's),
-// the inner solves of the refinement use CGS2: as stable, and three launches
-// per step instead of j + 3.
+// modified Gram-Schmidt, one pass per basis vector.  CGS2 is as stable
+// (orthogonal to rounding) and gives the same Hessenberg matrix to rounding,
+// in three launches per step instead of j + 3; the iterates and iteration
+// counts are compared with the oracle's MGS solver in the tests.
 //
 // Reductions: per-block partial sums, and the last block to finish (ticket
 // counter, no spinning) adds them in block order (deterministic).
@@ -103,7 +110,7 @@ __device__ __forceinline__ void rot_d(double &x, double &y, double c, double s) 
 
 template <typename T>
 __global__ void __launch_bounds__(kThreads) start_kernel(int64_t n, const T *__restrict__ r, ArnoldiCtrl *c,
-                                                         double tol, int iter_max, int first, double *part,
+                                                         double tol, int iter_max, int kind, double *part,
                                                          unsigned int *counter, ArnoldiStat *stat) {
     double v[1] = {0.0};
     for (int64_t e = (int64_t)blockIdx.x * kThreads + threadIdx.x; e < n; e += (int64_t)gridDim.x * kThreads) {
@@ -113,7 +120,7 @@ __global__ void __launch_bounds__(kThreads) start_kernel(int64_t n, const T *__r
     if (block_partials<1>(v, 1, part, counter) && threadIdx.x < 32) {
         const double beta = sqrt(warp_sum_partials(part, 0, threadIdx.x));
         if (threadIdx.x != 0) return;
-        if (first) {
+        if (kind == kStartSolve) {
             c->bn = beta;
             c->itn = 0;
             c->tol = tol;
@@ -124,7 +131,10 @@ __global__ void __launch_bounds__(kThreads) start_kernel(int64_t n, const T *__r
         c->g[0] = beta;
         c->k = 0;
         c->hnext = beta;
-        c->stop = isfinite(beta) ? (beta == 0.0 ? 1 : 0) : 3;
+        c->stop = !isfinite(beta) || !isfinite(c->bn) ? kStopNaN
+                  : c->bn == 0.0                      ? kStopZeroRhs
+                  : beta == 0.0                       ? kStopTol
+                                                      : 0;
         if (beta == 0.0) c->bea = 0.0;
         volatile ArnoldiStat *out = stat;
         out->stop = c->stop;
@@ -135,11 +145,12 @@ __global__ void __launch_bounds__(kThreads) start_kernel(int64_t n, const T *__r
     }
 }
 
-// out = w / hnext, unless the solve has stopped (or out is not needed)
+// out = V_k = w / hnext, unless the solve stopped before this step (k steps done)
 template <typename T>
-__global__ void scale_next_kernel(int64_t n, const T *__restrict__ w, T *__restrict__ out, const ArnoldiCtrl *c) {
+__global__ void scale_next_kernel(int64_t n, const T *__restrict__ w, T *__restrict__ out, const ArnoldiCtrl *c,
+                                  int k) {
     pdl_wait();
-    if (c->stop) return;
+    if (c->k != k || (k == 0 && c->stop)) return;
     const double inv = 1.0 / c->hnext;
     for (int64_t e = (int64_t)blockIdx.x * kThreads + threadIdx.x; e < n; e += (int64_t)gridDim.x * kThreads)
         out[e] = (T)((double)w[e] * inv);
@@ -259,9 +270,9 @@ __global__ void __launch_bounds__(kThreads) cgs_update_norm_kernel(int64_t n, T 
         const double bea = fabs(c->g[j + 1]) / c->bn;
         c->bea = bea;
         int stop = 0;
-        if (!finite || !isfinite(bea)) stop = 3;
-        else if (bea <= c->tol) stop = 1;
-        else if (c->itn >= c->iter_max) stop = 2;
+        if (!finite || !isfinite(bea)) stop = kStopNaN;
+        else if (bea <= c->tol) stop = kStopTol;
+        else if (c->itn >= c->iter_max) stop = kStopBudget;
         c->stop = stop;
         volatile ArnoldiStat *out = stat + j;
         out->stop = stop;
@@ -302,12 +313,12 @@ __global__ void vy_kernel(int64_t n, const T *__restrict__ V, const ArnoldiCtrl 
 }  // namespace
 
 template <typename T>
-cudaError_t launch_arnoldi_start(int64_t n, const T *r, T *V0, ArnoldiCtrl *c, double tol, int iter_max, int first,
-                                 double *part, unsigned int *counter, int max_blocks, ArnoldiStat *stat,
-                                 cudaStream_t st) {
+cudaError_t launch_arnoldi_start(int64_t n, const T *r, T *V0, ArnoldiCtrl *c, double tol, int iter_max,
+                                 ArnoldiStart kind, double *part, unsigned int *counter, int max_blocks,
+                                 ArnoldiStat *stat, cudaStream_t st) {
     const int nb = blocks_for(n, max_blocks);
-    start_kernel<T><<<nb, kThreads, 0, st>>>(n, r, c, tol, iter_max, first, part, counter, stat);
-    scale_next_kernel<T><<<nb, kThreads, 0, st>>>(n, r, V0, c);
+    start_kernel<T><<<nb, kThreads, 0, st>>>(n, r, c, tol, iter_max, kind, part, counter, stat);
+    scale_next_kernel<T><<<nb, kThreads, 0, st>>>(n, r, V0, c, 0);
     return cudaGetLastError();
 }
 
@@ -327,7 +338,7 @@ cudaError_t launch_arnoldi_orthogonalize(int64_t n, T *w, T *V, int j, int m, Ar
                        j, c, stat, part, counter);
     if (e == cudaSuccess && j + 1 < m)
         e = launch_pdl(scale_next_kernel<T>, dim3(nb), dim3(kThreads), 0, st, n, static_cast<const T *>(w),
-                       V + (int64_t)(j + 1) * n, static_cast<const ArnoldiCtrl *>(c));
+                       V + (int64_t)(j + 1) * n, static_cast<const ArnoldiCtrl *>(c), j + 1);
     return e;
 }
 
@@ -338,10 +349,12 @@ cudaError_t launch_arnoldi_combine(int64_t n, const T *V, ArnoldiCtrl *c, T *u, 
     return cudaGetLastError();
 }
 
-template cudaError_t launch_arnoldi_start<float>(int64_t, const float *, float *, ArnoldiCtrl *, double, int, int,
-                                                 double *, unsigned int *, int, ArnoldiStat *, cudaStream_t);
-template cudaError_t launch_arnoldi_start<double>(int64_t, const double *, double *, ArnoldiCtrl *, double, int, int,
-                                                  double *, unsigned int *, int, ArnoldiStat *, cudaStream_t);
+template cudaError_t launch_arnoldi_start<float>(int64_t, const float *, float *, ArnoldiCtrl *, double, int,
+                                                 ArnoldiStart, double *, unsigned int *, int, ArnoldiStat *,
+                                                 cudaStream_t);
+template cudaError_t launch_arnoldi_start<double>(int64_t, const double *, double *, ArnoldiCtrl *, double, int,
+                                                  ArnoldiStart, double *, unsigned int *, int, ArnoldiStat *,
+                                                  cudaStream_t);
 template cudaError_t launch_arnoldi_orthogonalize<float>(int64_t, float *, float *, int, int, ArnoldiCtrl *,
                                                          ArnoldiStat *, double *, unsigned int *, int, cudaStream_t);
 template cudaError_t launch_arnoldi_orthogonalize<double>(int64_t, double *, double *, int, int, ArnoldiCtrl *,

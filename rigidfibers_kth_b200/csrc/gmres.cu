@@ -89,105 +89,139 @@ cudaError_t Gmres<VT>::init(int64_t n, int m, cudaStream_t st) {
 }
 
 template <typename VT>
-cudaError_t Gmres<VT>::solve_device(const StopOp &A, const StopOp *P, const VT *b, VT *x, double tol, int max_iters,
-                                    GmresResult *res, const std::function<void()> &on_skipped_product) {
+cudaError_t Gmres<VT>::solve_device(const StopOp &A, const StopOp *P, const VT *b, VT *x, bool x_is_zero, double tol,
+                                    int max_iters, GmresResult *res, const std::function<void()> &on_skipped_product,
+                                    bool check_true) {
     *res = GmresResult();
     const int m = m_;
     if (!ctrl_ || m > kArnoldiMax) return cudaErrorInvalidValue;
     const int iterMax = max_iters > 0 ? max_iters : (int)n_;
     const int *stop = &ctrl_->stop;
     volatile ArnoldiStat *hs = hstat_;
-    RF_TRY(cudaMemsetAsync(x, 0, sizeof(VT) * n_, st_));
-    RF_TRY(launch_arnoldi_start<VT>(n_, b, V_, ctrl_, tol, iterMax, 1, cpart_, rb_.counter, rb_.max_blocks,
-                                    dstat_ + kArnoldiMax, st_));
-    res->launches += 3;
+    auto start = [&](const VT *r, ArnoldiStart kind) {
+        res->launches += 2;
+        return launch_arnoldi_start<VT>(n_, r, V_, ctrl_, tol, iterMax, kind, cpart_, rb_.counter, rb_.max_blocks,
+                                        dstat_ + kArnoldiMax, st_);
+    };
+    auto resid = [&](const VT *xv) -> cudaError_t {  // w_ = b - A xv
+        RF_TRY(A(xv, w_, nullptr));
+        res->matvecs++;
+        res->launches++;
+        return launch_bmr<VT>(n_, b, w_, st_);
+    };
+    // the first start records |b|, which every estimate and residual is relative to
+    RF_TRY(start(b, kStartSolve));
+    if (x_is_zero) {
+        RF_TRY(cudaMemsetAsync(x, 0, sizeof(VT) * n_, st_));
+    } else {
+        RF_TRY(resid(x));
+        RF_TRY(start(w_, kStartFrom));
+    }
     int last_stop = 0;
     for (;;) {
         // The start of a cycle may already stop the solve (zero or non-finite
         // residual).  Its outcome is read after the first step's event: steps
         // queued behind a stopped start return at once and leave their
         // outcome slots untouched.
-        bool ahead = false;  // a step was queued after the one that stopped
-        int queued = 0;
         int start_stop = -1;  // the start's outcome, once known
         auto read_start = [&] {
             if (start_stop < 0) start_stop = hs[kArnoldiMax].stop;
             return start_stop != 0;
         };
-        for (int j = 0; j < m; ++j) {
-            const VT *in = V_ + (size_t)j * n_;
-            if (P) {
-                RF_TRY((*P)(in, z_, stop));
-                res->launches++;
-                in = z_;
-            }
-            RF_TRY(A(in, w_, stop));
-            res->matvecs++;
-            RF_TRY(launch_arnoldi_orthogonalize<VT>(n_, w_, V_, j, m, ctrl_, dstat_, cpart_, rb_.counter,
-                                                    rb_.max_blocks, st_));
-            res->launches += 4;
-            RF_TRY(cudaEventRecord(step_ev_[j], st_));
-            ++queued;
-            if (j > 0) {
-                // step j is queued: now wait for step j - 1 (the GPU is busy with j)
-                RF_TRY(cudaEventSynchronize(step_ev_[j - 1]));
-                if (read_start()) break;
-                last_stop = hs[j - 1].stop;
-                res->iterations = hs[j - 1].itn;
-                res->backward_error = hs[j - 1].bea;
-                if (last_stop) {
-                    ahead = true;
-                    break;
+        for (int j = 0; j < m;) {
+            bool ahead = false;  // a step was queued after the one that stopped
+            int queued = 0, done = -1;
+            for (; j < m; ++j) {
+                const VT *in = V_ + (size_t)j * n_;
+                if (P) {
+                    RF_TRY((*P)(in, z_, stop));
+                    res->launches++;
+                    in = z_;
+                }
+                RF_TRY(A(in, w_, stop));
+                res->matvecs++;
+                RF_TRY(launch_arnoldi_orthogonalize<VT>(n_, w_, V_, j, m, ctrl_, dstat_, cpart_, rb_.counter,
+                                                        rb_.max_blocks, st_));
+                res->launches += 4;
+                RF_TRY(cudaEventRecord(step_ev_[j], st_));
+                ++queued;
+                if (queued > 1) {
+                    // step j is queued: now wait for step j - 1 (the GPU is busy with j)
+                    RF_TRY(cudaEventSynchronize(step_ev_[j - 1]));
+                    if (read_start()) break;
+                    done = j - 1;
+                    if (hs[done].stop) {
+                        ahead = true;
+                        break;
+                    }
                 }
             }
-        }
-        if (start_stop <= 0 && !ahead) {
-            RF_TRY(cudaEventSynchronize(step_ev_[m - 1]));
-            if (!read_start()) {
-                last_stop = hs[m - 1].stop;
-                res->iterations = hs[m - 1].itn;
-                res->backward_error = hs[m - 1].bea;
+            if (start_stop <= 0 && !ahead) {
+                RF_TRY(cudaEventSynchronize(step_ev_[m - 1]));
+                if (!read_start()) done = m - 1;
             }
-        }
-        if (start_stop > 0) {
-            // every step of this cycle returned at once
-            for (int q = 0; q < queued; ++q) {
-                res->matvecs--;
+            if (start_stop > 0) {
+                // every step of this cycle returned at once
+                for (int q = 0; q < queued; ++q) {
+                    res->matvecs--;
+                    if (on_skipped_product) on_skipped_product();
+                }
+                if (start_stop == kStopZeroRhs) RF_TRY(cudaMemsetAsync(x, 0, sizeof(VT) * n_, st_));
+                res->info = start_stop == kStopNaN ? kInfoNaN : 0;
+                return cudaSuccess;
+            }
+            last_stop = hs[done].stop;
+            res->iterations = hs[done].itn;
+            res->backward_error = hs[done].bea;
+            if (ahead) {
+                res->matvecs--;  // the queued step's product returned at once
                 if (on_skipped_product) on_skipped_product();
             }
-            res->info = start_stop == 3 ? kInfoNaN : 0;
-            return cudaSuccess;
-        }
-        if (ahead) {
-            res->matvecs--;  // the queued step's product returned at once
-            if (on_skipped_product) on_skipped_product();
-        }
-        if (last_stop == 3) {
-            res->info = kInfoNaN;
-            return cudaSuccess;
-        }
-        // x += P (V y) over the steps of this cycle
-        RF_TRY(launch_arnoldi_combine<VT>(n_, V_, ctrl_, u_, st_));
-        res->launches += 2;
-        const VT *upd = u_;
-        if (P) {
-            RF_TRY((*P)(u_, z_, nullptr));
-            upd = z_;
+            if (last_stop == kStopNaN) {
+                res->info = kInfoNaN;
+                return cudaSuccess;
+            }
+            // xcur = x + P (V y) over the steps of this cycle
+            RF_TRY(launch_arnoldi_combine<VT>(n_, V_, ctrl_, u_, st_));
+            res->launches += 2;
+            const VT *upd = u_;
+            if (P) {
+                RF_TRY((*P)(u_, z_, nullptr));
+                upd = z_;
+                res->launches++;
+            }
+            VT *xnew = last_stop && check_true ? xcur_ : x;
+            RF_TRY(launch_add<VT>(n_, x, upd, xnew, st_));
             res->launches++;
-        }
-        RF_TRY(launch_add<VT>(n_, x, upd, x, st_));
-        res->launches++;
-        if (last_stop) {
-            res->info = last_stop == 1 ? 0 : kInfoBudget;
-            return cudaSuccess;
+            if (!last_stop) break;  // the end of the cycle
+            if (!check_true) {
+                res->info = last_stop == kStopTol ? 0 : kInfoBudget;
+                return cudaSuccess;
+            }
+            // the estimate met the tolerance (or the budget is spent): the true residual decides
+            RF_TRY(resid(xcur_));
+            double tn, bn;
+            RF_TRY(launch_dot<VT>(n_, w_, w_, hcol_, rb_, st_));
+            res->launches++;
+            RF_TRY(cudaMemcpyAsync(hpin_ + 1, &ctrl_->bn, sizeof(double), cudaMemcpyDeviceToHost, st_));
+            RF_TRY(fetch(hcol_, &tn, 1));
+            bn = hpin_[1];
+            res->backward_error = std::sqrt(tn) / bn;
+            if (res->backward_error <= tol || res->iterations >= iterMax) {
+                RF_TRY(cudaMemcpyAsync(x, xcur_, sizeof(VT) * n_, cudaMemcpyDeviceToDevice, st_));
+                RF_TRY(cudaStreamSynchronize(st_));
+                res->info = res->backward_error <= tol ? 0 : kInfoBudget;
+                return cudaSuccess;
+            }
+            // not there yet: this cycle goes on with step done + 1 (its basis
+            // vector is in place), or restarts if that was its last step
+            RF_TRY(cudaMemsetAsync(&ctrl_->stop, 0, sizeof(int), st_));
+            j = done + 1;
+            if (j == m) RF_TRY(cudaMemcpyAsync(x, xcur_, sizeof(VT) * n_, cudaMemcpyDeviceToDevice, st_));
         }
         // restart from the residual of the updated x
-        RF_TRY(A(x, w_, nullptr));
-        res->matvecs++;
-        RF_TRY(launch_bmr<VT>(n_, b, w_, st_));
-        RF_TRY(launch_arnoldi_start<VT>(n_, w_, V_, ctrl_, tol, iterMax, 0, cpart_, rb_.counter, rb_.max_blocks,
-                                        dstat_ + kArnoldiMax, st_));
-        res->launches += 4;
+        RF_TRY(resid(x));
+        RF_TRY(start(w_, kStartFrom));
     }
 }
 

@@ -7,7 +7,7 @@
 // optional (the residual keeps its meaning).  Krylov vectors live on the
 // device in VT (double or float); the Hessenberg matrix, rotations and the
 // least-squares solve are FP64 on the host (a few hundred flops per step);
-// solve_device keeps them on the device (arnoldi.cu).
+// solve_device keeps them on the device (arnoldi.cu) with the same flow.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -46,16 +46,16 @@ class Gmres {
     // solves of iterative refinement, whose caller recomputes the residual).
     cudaError_t solve(const Op &A, const Op *P, const VT *b, VT *x, bool x_is_zero, double tol, int max_iters,
                       GmresResult *res, bool check_true = true);
-    // Inner solve of the refinement, controlled on the device (arnoldi.cu):
-    // x = 0 initially, stop on the Arnoldi estimate <= tol or the budget,
-    // CGS2 orthogonalisation.  The host queues each step before it learns
-    // whether the previous one stopped (the first steps of a cycle also
-    // before it learns whether the cycle's start stopped); a step queued
-    // after the stop runs as empty launches, and `on_skipped_product` is
-    // called once for each such product (the caller's product timer drops
-    // it).  Needs m <= kArnoldiMax.
-    cudaError_t solve_device(const StopOp &A, const StopOp *P, const VT *b, VT *x, double tol, int max_iters,
-                             GmresResult *res, const std::function<void()> &on_skipped_product);
+    // The same solve controlled on the device (arnoldi.cu): the host queues
+    // each step before it learns whether the previous one stopped (the first
+    // steps of a cycle also before it learns whether the cycle's start
+    // stopped); a step queued after the stop runs as empty launches, and
+    // `on_skipped_product` is called once for each such product (the caller's
+    // product timer drops it).  CGS2 orthogonalisation.  Needs
+    // m <= kArnoldiMax.
+    cudaError_t solve_device(const StopOp &A, const StopOp *P, const VT *b, VT *x, bool x_is_zero, double tol,
+                             int max_iters, GmresResult *res, const std::function<void()> &on_skipped_product,
+                             bool check_true);
     int restart() const { return m_; }
 
    private:

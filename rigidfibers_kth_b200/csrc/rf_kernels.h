@@ -270,8 +270,15 @@ struct ArnoldiCtrl {
     int k;             // Arnoldi steps of the current cycle
     int itn;           // steps over all cycles
     int iter_max;      // step budget
-    int stop;          // 0 running, 1 estimate <= tol, 2 budget spent, 3 non-finite value
+    int stop;          // 0 running, else one of the outcomes below
 };
+constexpr int kStopTol = 1;       // estimate <= tol (or a zero residual)
+constexpr int kStopBudget = 2;    // step budget spent
+constexpr int kStopNaN = 3;       // non-finite value
+constexpr int kStopZeroRhs = 4;   // |b| = 0 at a cycle's start
+// What a cycle starts from: the solve's right-hand side (records |b|, the
+// tolerance and the budget) or the residual of a current iterate.
+enum ArnoldiStart { kStartSolve, kStartFrom };
 // One step's outcome as the host sees it (host-mapped memory written by the device).
 struct ArnoldiStat {
     int stop;
@@ -279,18 +286,19 @@ struct ArnoldiStat {
     double bea;
 };
 // Start of a cycle: beta = |r| (r the cycle's residual); g = (beta, 0, ...),
-// k = 0, stop = 0 (1 if beta = 0, 3 if not finite), written to *stat
-// (host-mapped) too; with first != 0 also bn = beta, itn = 0 and the
+// k = 0, stop = 0 (or the outcome of a zero or non-finite residual), written
+// to *stat (host-mapped) too; kStartSolve also sets bn = beta, itn = 0 and the
 // tolerance and budget; then V_0 = r / beta.
 template <typename T>
-cudaError_t launch_arnoldi_start(int64_t n, const T *r, T *V0, ArnoldiCtrl *c, double tol, int iter_max, int first,
-                                 double *part, unsigned int *counter, int max_blocks, ArnoldiStat *stat,
-                                 cudaStream_t st);
+cudaError_t launch_arnoldi_start(int64_t n, const T *r, T *V0, ArnoldiCtrl *c, double tol, int iter_max,
+                                 ArnoldiStart kind, double *part, unsigned int *counter, int max_blocks,
+                                 ArnoldiStat *stat, cudaStream_t st);
 // Step j after w = A z: two classical Gram-Schmidt passes against V_0..V_j
 // (dots; update and dots; update and norm), then the Givens update of column
 // j, the stop test, the step's outcome into stat[j] (host-mapped), and
-// V_{j+1} = w / |w| unless the solve stopped or j + 1 = m.  Every kernel
-// returns at once when the solve has stopped before it.
+// V_{j+1} = w / |w| unless j + 1 = m (also when step j stops the solve: its
+// cycle goes on if the true residual is still above the tolerance).  Every
+// kernel returns at once when the solve has stopped before this step.
 template <typename T>
 cudaError_t launch_arnoldi_orthogonalize(int64_t n, T *w, T *V, int j, int m, ArnoldiCtrl *c, ArnoldiStat *stat,
                                          double *part, unsigned int *counter, int max_blocks, cudaStream_t st);

@@ -1,0 +1,61 @@
+"""The device-controlled GMRES (restart lengths up to 16) against the oracle's
+solver on the same matrix: iterates, iteration counts, budget, cold and warm
+starts, and the host-controlled solver above that length."""
+import numpy as np
+import pytest
+
+import rigidfibers_kth_b200 as rf
+from oracle import rfo
+
+pytestmark = pytest.mark.gpu
+
+
+def system(M, **kw):
+    pos, ori = rf.generate_layout(M, "uniform", (M / 8.0) ** (1 / 3), 0.2, seed=40 + M)
+    sim = rf.Simulation(rf.Configuration(rf.FiberParams(slenderness=1e-3, **kw), pos, ori))
+    sim.assemble_system()
+    return sim, np.array(sim.matrix(), order="F"), sim.rhs()
+
+
+# restart 1 (every cycle one step), the reference's 10, the last
+# device-controlled length and the first host-controlled one; 3 iterations
+# end inside a cycle, on its last step and before convergence
+@pytest.mark.parametrize("restart,tol,budget", [(1, 1e-4, 400), (3, 1e-8, 3), (10, 1e-10, 300), (10, 1e-13, 300),
+                                                (16, 1e-10, 16), (16, 1e-12, 300), (17, 1e-12, 300)])
+@pytest.mark.parametrize("M", [1, 2, 37])
+def test_iterates_match_oracle(M, restart, tol, budget):
+    sim, A, b = system(M, gmres_restart=restart, gmres_tol=tol, gmres_max_iters=budget)
+    with sim:
+        sim.solve_system()
+        x, st = sim.coeffs(), sim.solve_stats()
+    x_o, info, iters, be = rfo.solve_gmres(A, b, restart=restart, max_iters=budget, tol=tol)
+    assert st["converged"] == (info == 0)
+    # both end on a residual within a few units of rounding of each other; the
+    # count may move by one where the estimate meets 1e-13 at that level
+    assert abs(st["iterations"] - iters) <= (1 if tol < 1e-12 else 0)
+    assert np.abs(x - x_o).max() <= 1e-10 * max(1e-30, np.abs(x_o).max())
+
+
+@pytest.mark.parametrize("precision,tol", [(rf.PREC_FP64, 1e-10), (rf.PREC_FP32, 1e-5)])
+def test_warm_start_zero_rhs_and_true_residual(precision, tol):
+    """A start from the solution ends at once; the residual reported is the
+    true one; without external force b = 0 and x = 0 whatever the start."""
+    sim, A, b = system(37, gmres_tol=tol, gmres_max_iters=300, precision=precision)
+    with sim:
+        assert sim.solve_system() == 0
+        x, st = sim.coeffs(), sim.solve_stats()
+        true = np.linalg.norm(b - A @ x) / np.linalg.norm(b)
+        # the device forms the residual from sums of n = 555 products in the
+        # storage precision: n * eps of |A| |x| ~ 3 |b| on top
+        eps = 2.0 ** -53 if precision == rf.PREC_FP64 else 2.0 ** -24
+        assert st["residual"] <= tol and abs(st["residual"] - true) <= 3 * 555 * eps
+        its = st["iterations"]
+        assert sim.solve_system() == 0  # from x
+        assert sim.solve_stats()["iterations"] <= 2 < its
+    sim, A, b = system(5, gmres_tol=tol, precision=precision, external_force=(0.0, 0.0, 0.0))
+    with sim:
+        z = np.zeros(15)
+        sim.set_history(z, z + 1.0, z, z, np.ones(75))
+        assert np.abs(b).max() == 0.0
+        assert sim.solve_system() == 0
+        assert np.abs(sim.coeffs()).max() == 0.0
