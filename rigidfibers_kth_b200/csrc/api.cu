@@ -427,6 +427,11 @@ rf_status rf_create(const rf_params *p, const double *positions, const double *o
     h->asm_chunks = (M + h->asm_chunk - 1) / h->asm_chunk;
     h->vel_chunk = h->asm_chunk;
     h->vel_chunks = h->asm_chunks;
+    h->asm64 = prec == RF_PREC_FP64 && p->use_analytical_integration != 0 && rf::assemble64_supported(N);
+    if (h->asm64) {
+        h->asm_chunks = rf::assemble64_chunks(M, h->sm_count);
+        h->asm_chunk = (M + h->asm_chunks - 1) / h->asm_chunks;
+    }
     CKC(dalloc(&h->b, h->n), "alloc b");
     CKC(dalloc(&h->x, h->n), "alloc x");
     CKC(cudaMemset(h->x, 0, h->n * 8), "memset x");
@@ -666,8 +671,11 @@ rf_status rf_assemble_system(rf_handle *h) {
         // near_field_c >= 1e30 keeps every integral in FP64 for the mixed paths
         const int pmode = (prec == RF_PREC_FP64 || (prec != RF_PREC_FP32 && a.near_c >= 1e30)) ? rf::kPModeFP64
                                                                                               : rf::kPModeMixed;
-        CK(h, rf::launch_assemble(a, h->p.use_analytical_integration == 0, pmode, h->asm_chunks, h->stream),
-           "assemble kernel");
+        if (h->asm64)
+            CK(h, rf::launch_assemble64(a, h->asm_chunks, h->stream), "assemble kernel");
+        else
+            CK(h, rf::launch_assemble(a, h->p.use_analytical_integration == 0, pmode, h->asm_chunks, h->stream),
+               "assemble kernel");
         CK(h, rf::launch_reduce_chunks(h->bpart, h->asm_chunks, h->n_loc, h->n_loc, h->b + 3LL * h->N * h->t0,
                                        h->stream),
            "rhs reduction");

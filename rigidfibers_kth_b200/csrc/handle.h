@@ -50,6 +50,7 @@ struct rf_handle {
     double *x = nullptr;       // coefficients (warm start for the next solve)
     double *bpart = nullptr;   // [nchunks][n]
     int asm_chunks = 1, asm_chunk = 1;
+    bool asm64 = false;        // FP64 analytic assembly by autonomous warps (assemble64.cu)
     int vel_chunks = 1, vel_chunk = 1;
     double *velpart = nullptr; // [vel_chunks][6M]
     double *mfpart = nullptr;  // [vel_chunks][n] matrix-free product partials, made at its first use

@@ -61,56 +61,118 @@ __device__ __forceinline__ double fadd(double a, double b) { return __dadd_rn(a,
 __device__ __forceinline__ double fsub(double a, double b) { return __dsub_rn(a, b); }
 __device__ __forceinline__ double fdiv(double a, double b) { return __ddiv_rn(a, b); }
 
+// x / OM for a small integer OM, correctly rounded: q = RN(x r), r = RN(1/OM),
+// then one step with the exact remainder, RN(q + (x - q OM) r) (Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000 processor",
+// 1990).  q is within two units of the quotient, so the remainder is a
+// multiple of q's unit below 2^6 units and the fused multiply-add forms it
+// exactly; the corrected sum is off by less than 2^-50 units before its
+// rounding, and x / OM (OM = 2^k times an odd m) is either representable or at
+// least 1/(2m) units away from a rounding boundary.  Three instructions for
+// the general division's dozen.
+template <int OM>
+__device__ __forceinline__ double div_const(double x) {
+    constexpr int m = OM < 0 ? -OM : OM;
+    constexpr double r = 1.0 / OM;
+    const double q = __dmul_rn(x, r);
+    if constexpr ((m & (m - 1)) == 0) return q;  // a power of two: exact
+    else return __fma_rn(__fma_rn(-q, (double)OM, x), r, q);
+}
+
+// 1/x and 1/sqrt(x) of a positive normal x, within two units: the hardware's
+// approximation y (relative error below 2^-19), then the series in e = 1 - x y
+// (1/x = y / (1 - e)) or e = 1 - x y^2 (1/sqrt(x) = y (1 - e)^(-1/2)) up to
+// e^2; the first neglected terms are e^3 and 5/16 e^3.  Three and five FP64
+// operations and no branch.
+__device__ __forceinline__ double rcp_pos(double x) {
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-x, y, 1.0);
+    return fma(y, fma(e, e, e), y);
+}
+__device__ __forceinline__ double rsqrt_pos(double x) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-x * y, y, 1.0);
+    return fma(y * e, fma(0.375, e, 0.5), y);
+}
+// a / b from y = 1/b (within two units), and sqrt(x): one correction with the
+// exact remainder (Markstein 1990, as div_const), off by less than 2^-50 units
+// before its rounding: the correctly rounded value except where the quotient
+// or root lies that close to a rounding boundary.  The compiler's division and
+// square root branch to a path for subnormal and special operands, so that the
+// ten divisions of the closed forms run one after the other; these interleave,
+// and quotients of one denominator share its reciprocal.  A zero or infinite
+// operand gives NaN (the reference's formulas are singular there).
+__device__ __forceinline__ double div_by(double a, double b, double y) {
+    const double q = __dmul_rn(a, y);
+    return __fma_rn(__fma_rn(-q, b, a), y, q);
+}
+__device__ __forceinline__ double sqrt_pos(double x) {
+    const double y = rsqrt_pos(x);
+    const double g = __dmul_rn(x, y);
+    return __fma_rn(__fma_rn(-g, g, x), 0.5 * y, g);
+}
+
+// Steps n .. K-1 of the reference's forward recursion (Int_analytical.f90:
+// 123-136, 172-176, 197-200) in its operation order; Fortran nn = n + 1.
+template <int n, int K>
+struct ForwardStep {
+    __device__ __forceinline__ static void run(double b, double c, double ue, double ub, double *I, double *J,
+                                               double *S) {
+        if constexpr (n < K) {
+            const double t1 = div_const<-n>(ue);
+            const double t2 = div_const<-n>(n % 2 == 1 ? ub : -ub);  // sb**(ii-2) ub
+            const double t3 = fmul(div_const<-n>(fmul(0.5 - n, b)), I[n - 1]);
+            const double t4 = fmul(div_const<-n>(fmul(n - 1.0, c)), I[n - 2]);
+            I[n] = fadd(fsub(fsub(t2, t1), t3), t4);
+            J[n] = fsub(fsub(I[n - 2], fmul(b, J[n - 1])), fmul(c, J[n - 2]));
+            S[n] = fsub(fsub(J[n - 2], fmul(b, S[n - 1])), fmul(c, S[n - 2]));
+            ForwardStep<n + 1, K>::run(b, c, ue, ub, I, J, S);
+        }
+    }
+};
+
 template <int N>
 __device__ __forceinline__ void moments_fp64(double b, double c, double *I, double *J, double *S) {
     constexpr int K = N + 3;
     // Int_analytical.f90:96-102
-    const double ue = sqrt(fadd(fadd(1.0, b), c));
-    const double ub = sqrt(fadd(fsub(1.0, b), c));
+    const double ue = sqrt_pos(fadd(fadd(1.0, b), c));
+    const double ub = sqrt_pos(fadd(fsub(1.0, b), c));
     const double te = fadd(1.0, fmul(0.5, b));
     const double tb = fadd(-1.0, fmul(0.5, b));
     const double d = fsub(c, fmul(fmul(0.25, b), b));
+    const double rue = rcp_pos(ue), rub = rcp_pos(ub);
+    const double j1c = fadd(div_by(-1.0, ue, rue), div_by(1.0, ub, rub));
     // :113-114
     I[0] = fsub(log(fabs(fadd(fadd(2.0, b), fmul(2.0, ue)))), log(fabs(fadd(fadd(-2.0, b), fmul(2.0, ub)))));
     I[1] = fsub(fsub(ue, ub), fmul(fmul(0.5, b), I[0]));
-    // :162-170
+    // :162-170, 189-196
     if (d < 1e-14) {
         const double e1 = fadd(1.0, fmul(b, 0.5)), e2 = fadd(-1.0, fmul(b, 0.5));  // b/2 is exact
         J[0] = fadd(fdiv(-1.0, fmul(2.0, fmul(e1, e1))), fdiv(1.0, fmul(2.0, fmul(e2, e2))));
-    } else {
-        J[0] = fsub(fdiv(te, fmul(d, ue)), fdiv(tb, fmul(d, ub)));
-    }
-    J[1] = fsub(fadd(fdiv(-1.0, ue), fdiv(1.0, ub)), fmul(fmul(b, 0.5), J[0]));
-    // :189-196
-    if (d < 1e-14) {
+        J[1] = fsub(j1c, fmul(fmul(b, 0.5), J[0]));
         const double p = fadd(2.0, b), m = fadd(-2.0, b);
         const double p2 = fmul(p, p), m2 = fmul(m, m);
         S[0] = fadd(fdiv(-4.0, fmul(p2, p2)), fdiv(4.0, fmul(m2, m2)));
         S[1] = fsub(fadd(fdiv(-8.0, fmul(3.0, fmul(p2, p))), fdiv(8.0, fmul(3.0, fmul(m2, m)))),
                     fmul(fmul(b, 0.5), S[0]));
     } else {
-        const double ue3 = fmul(fmul(ue, ue), ue), ub3 = fmul(fmul(ub, ub), ub);
-        const double d6 = fmul(6.0, d);
-        S[0] = fadd(fsub(fdiv(fadd(2.0, b), fmul(d6, ue3)), fdiv(fadd(-2.0, b), fmul(d6, ub3))),
-                    fmul(fdiv(2.0, fmul(3.0, d)), J[0]));
-        S[1] = fsub(fadd(fdiv(-fadd(b, fmul(2.0, c)), fmul(d6, ue3)), fdiv(fadd(-b, fmul(2.0, c)), fmul(d6, ub3))),
-                    fmul(fdiv(b, fmul(3.0, d)), J[0]));
+        const double due = fmul(d, ue), dub = fmul(d, ub), d3 = fmul(3.0, d), d6 = fmul(6.0, d);
+        const double de = fmul(d6, fmul(fmul(ue, ue), ue)), db = fmul(d6, fmul(fmul(ub, ub), ub));
+        // the reciprocals of the five products of d, ue and ub from theirs
+        const double rd = rcp_pos(d), r6 = rd * (1.0 / 6.0);
+        const double rde = r6 * rue * rue * rue, rdb = r6 * rub * rub * rub, rd3 = rd * (1.0 / 3.0);
+        J[0] = fsub(div_by(te, due, rd * rue), div_by(tb, dub, rd * rub));
+        J[1] = fsub(j1c, fmul(fmul(b, 0.5), J[0]));
+        S[0] = fadd(fsub(div_by(fadd(2.0, b), de, rde), div_by(fadd(-2.0, b), db, rdb)),
+                    fmul(div_by(2.0, d3, rd3), J[0]));
+        S[1] = fsub(fadd(div_by(-fadd(b, fmul(2.0, c)), de, rde), div_by(fadd(-b, fmul(2.0, c)), db, rdb)),
+                    fmul(div_by(b, d3, rd3), J[0]));
     }
     if (c < 10.0) {
         // forward recursion, :123-136, 172-176, 197-200
-#pragma unroll
-        for (int n = 2; n < K; ++n) {
-            const double nn = n + 1.0;                     // Fortran nn
-            const double om = 1.0 - nn;
-            const double sbp = (n % 2 == 1) ? 1.0 : -1.0;  // sb**(ii-2)
-            const double t1 = fdiv(ue, om);
-            const double t2 = fdiv(fmul(sbp, ub), om);
-            const double t3 = fmul(fdiv(fmul(0.5 - (nn - 1.0), b), om), I[n - 1]);
-            const double t4 = fmul(fdiv(fmul(nn - 2.0, c), om), I[n - 2]);
-            I[n] = fadd(fsub(fsub(t2, t1), t3), t4);
-            J[n] = fsub(fsub(I[n - 2], fmul(b, J[n - 1])), fmul(c, J[n - 2]));
-            S[n] = fsub(fsub(J[n - 2], fmul(b, S[n - 1])), fmul(c, S[n - 2]));
-        }
+        ForwardStep<2, K>::run(b, c, ue, ub, I, J, S);
     } else {
         // backward recursion from n = 27 (:137-157, 177-183, 201-206); stable, so
         // folded constants and fused arithmetic are used here
@@ -130,6 +192,107 @@ __device__ __forceinline__ void moments_fp64(double b, double c, double *I, doub
             i2 = i1; i1 = in; j2 = j1; j1 = jn; s2 = s1; s1 = sn;
         }
     }
+}
+
+// ---------------------------------------------------------------------------
+// FP64 far points.  The kernels that need the moments only as
+// u_p = I_p + 2 eps^2 J_p (p = 0..N) and v_p = J_p - 6 eps^2 S_p (p = 0..N+2)
+// take a far point (10 <= c < 4096, outside a cone about the source axis) through the
+// backward recursion alone, run down to n = 0: the three-term relations that
+// the reference uses for n >= 2 hold at n = 0, 1 too.  That leaves out the two
+// logarithms and ten divisions of the closed forms: about 260 FP64
+// instructions for the reference's 450.  Where the lines lie: below c = 10 the
+// reference recurs forward and amplifies every rounding, so those points
+// follow its operation order (moments_fp64); in the cone (d = c - b^2/4 below
+// kAxisRatio c: 1 point in 2000 of an isotropic suspension; kAxisRatioNear c
+// while c < 16) its closed forms lose digits to the divisions by d and its
+// start at n = 27 leaves up to 2e-9 |J_0|, and parity with it is kept; from 64
+// half-lengths on its closed forms' cancellation (a relative error that grows
+// like c, 4e-9 at c = 10^6) would show against the recursion likewise.
+// The start (far_top): zero starting values reach n <= 7 damped by c^(-n/2)
+// times a polynomial in n, and an even start is closer than an odd one, so it
+// falls with c.  Relative to J_0, 40-digit evaluation, n <= 7, at the lower
+// end of every range: J_n within 7e-13 for |b| up to 0.9 of its largest value
+// and 4e-12 at the edge of the cone; the start at 27 leaves 3e-11 at |b| = 0.9
+// of its largest value at c = 10.
+constexpr double kFarC = 10.0;
+constexpr double kFarMaxC = 4096.0;
+constexpr double kAxisRatio = 1e-3, kAxisRatioNear = 1e-2;
+__device__ __forceinline__ bool far_point(double b, double c) {
+    return c >= kFarC && c < kFarMaxC && fma(-0.25 * b, b, c) >= (c < 16.0 ? kAxisRatioNear : kAxisRatio) * c;
+}
+__device__ __forceinline__ int far_top(float c) {
+    return 16 + 2 * ((c < 150.f) + (c < 80.f) + (c < 48.f) + (c < 30.f) + (c < 20.f) + (c < 16.f) + (c < 13.f));
+}
+
+// Step n: I_n = -(1 + r/2) (b/c) I_{n+1} - (1 + r) (1/c) I_{n+2} + r w, r =
+// 1/(n+1), w = (ue -+ ub)/c.  r comes from a table in shared memory for the
+// steps above kFarTail, which run as a loop (a fully unrolled recursion
+// exceeds the instruction cache that a scheduler's warps share).
+constexpr int kFarTail = 8;
+constexpr int kFarTop = 30;
+constexpr int kFarCoef = kFarTop - kFarTail;
+// entry t of the table: r of step kFarTail + 1 + t
+__device__ __forceinline__ double far_coef(int t) { return 1.0 / (kFarTail + 2.0 + t); }
+
+struct FarState {
+    double nicb, hicb, nic, wp, wm, ic;      // -b/c, -b/(2c), -1/c, (ue - ub)/c, (ue + ub)/c, 1/c
+    double i1, i2, j1, j2, s1, s2;           // I, c J, c^2 S at n + 1, n + 2
+    __device__ __forceinline__ void step(double r, double w) {
+        const double in = fma(fma(r, hicb, nicb), i1, fma(fma(r, nic, nic), i2, r * w));
+        const double jn = fma(nicb, j1, fma(nic, j2, in));
+        const double sn = fma(nicb, s1, fma(nic, s2, jn));
+        i2 = i1; i1 = in; j2 = j1; j1 = jn; s2 = s1; s1 = sn;
+    }
+};
+
+// the last steps, n .. 0; u_n and v_n to out as soon as they are formed
+template <int N, int n, typename OUT>
+__device__ __forceinline__ void far_tail(FarState &f, double e2, double e6, const OUT &out) {
+    if constexpr (n >= 0) {
+        f.step(1.0 / (n + 1.0), n % 2 == 1 ? f.wp : f.wm);
+        if constexpr (n <= N) out.u(n, fma(e2, f.j1, f.i1));
+        if constexpr (n <= N + 2) out.v(n, fma(f.ic, f.j1, e6 * f.s1));
+        far_tail<N, n - 1>(f, e2, e6, out);
+    }
+}
+
+// u_p and v_p of a far point, from the start its own c asks for: a point's
+// moments do not depend on the points beside it.  coef: the table above.
+// ue ub = sqrt((1 + c)^2 - b^2) and (ue + ub)^2 = 2 (1 + c + ue ub); ue - ub =
+// 2b / (ue + ub).
+template <int N, typename OUT>
+__device__ __forceinline__ void moments_far_fp64(double b, double c, double eps2, const double *coef, const OUT &out) {
+    const double t = 1.0 + c, pp = fma(t, t, -b * b);
+    const double us2 = 2.0 * fma(pp, rsqrt_pos(pp), t);
+    const double ius = rsqrt_pos(us2);
+    FarState f;
+    f.ic = rcp_pos(c);
+    f.nic = -f.ic;
+    f.nicb = f.nic * b;
+    f.hicb = 0.5 * f.nicb;
+    f.wp = -2.0 * f.nicb * ius;
+    f.wm = us2 * ius * f.ic;
+    f.i1 = f.i2 = f.j1 = f.j2 = f.s1 = f.s2 = 0.0;
+    const double *k = coef + (far_top((float)c) - kFarTail - 2);  // of the odd step below the start
+#pragma unroll 1
+    for (; k >= coef; k -= 2) {
+        f.step(k[1], f.wm);  // even n
+        f.step(k[0], f.wp);  // odd n
+    }
+    const double e2 = 2.0 * eps2 * f.ic;
+    far_tail<N, kFarTail>(f, e2, -3.0 * e2 * f.ic, out);
+}
+
+// The same families of any point from the reference's moments.
+template <int N, typename OUT>
+__device__ __forceinline__ void moments_near_uv(double b, double c, double eps2, const OUT &out) {
+    double I[N + 3], J[N + 3], S[N + 3];
+    moments_fp64<N>(b, c, I, J, S);
+#pragma unroll
+    for (int p = 0; p <= N; ++p) out.u(p, fma(2.0 * eps2, J[p], I[p]));
+#pragma unroll
+    for (int p = 0; p <= N + 2; ++p) out.v(p, fma(-6.0 * eps2, S[p], J[p]));
 }
 
 // First index of the FP32 backward recursion.  Its starting values

@@ -90,6 +90,10 @@ struct AsmArgs {
 };
 
 cudaError_t launch_assemble(const AsmArgs &a, bool numeric, int pmode, int nchunks, cudaStream_t st);
+// FP64 matrix, analytic integral, N <= 5 (assemble64.cu): the same outputs
+bool assemble64_supported(int N);
+int assemble64_chunks(int M, int sm_count);
+cudaError_t launch_assemble64(const AsmArgs &a, int nchunks, cudaStream_t st);
 
 // Mixed-precision assembly split into far pairs (FP32) and near pairs (FP64),
 // analytic integration, N <= 5 (assemble_split.cu).
