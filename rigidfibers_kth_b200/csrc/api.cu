@@ -395,10 +395,9 @@ rf_status rf_create(const rf_params *p, const double *positions, const double *o
     }
     // assembly chunking (from the whole system's targets also for a
     // row-block shard, so that its right-hand side sums the same source
-    // chunks in the same order).  The FP64 assembly runs CTAs of 4 targets,
-    // 4 resident per SM, the velocity kernel CTAs of 8 targets, 2 per SM: in
-    // both the grid takes about rounds x sources per CTA, rounds =
-    // (M / 4) x chunks / (4 SMs' worth of slots).  From a first guess of
+    // chunks in the same order).  The tile assembly runs CTAs of 4 targets,
+    // 4 resident per SM: the grid takes about rounds x sources per CTA, rounds
+    // = (M / 4) x chunks / (4 SMs' worth of slots).  From a first guess of
     // about 8 CTAs of 8 targets per SM, the sources per CTA (within a factor
     // 4 below, but not below 16, and 2 above) that minimise that product;
     // ties: the larger share.  At M = 4000 on 148 SMs: 13 chunks of 308
@@ -425,8 +424,8 @@ rf_status rf_create(const rf_params *p, const double *positions, const double *o
     }
     h->asm_chunk = (M + chunks - 1) / chunks;
     h->asm_chunks = (M + h->asm_chunk - 1) / h->asm_chunk;
-    h->vel_chunk = h->asm_chunk;
-    h->vel_chunks = h->asm_chunks;
+    h->vel_chunks = rf::pair_sum_chunks(M, h->sm_count);
+    h->vel_chunk = (M + h->vel_chunks - 1) / h->vel_chunks;
     h->asm64 = prec == RF_PREC_FP64 && p->use_analytical_integration != 0 && rf::assemble64_supported(N);
     if (h->asm64) {
         h->asm_chunks = rf::assemble64_chunks(M, h->sm_count);

@@ -114,8 +114,8 @@ __global__ void __launch_bounds__(kWarps * 32, 4) assemble64_kernel(AsmArgs a) {
     double *s_pv = reinterpret_cast<double *>(smem_raw);               // kMaxLQ
     RowTab *s_row = reinterpret_cast<RowTab *>(s_pv + kMaxLQ);          // NL block rows, then 2 panel rows
     double *s_leg = reinterpret_cast<double *>(s_row + NL + 2);         // NL x 3: coefficients of p = m, m-2, m-4
-    double *s_far = s_leg + NL * 3;                                     // kFarCoef
-    double *s_warp = s_far + kFarCoef;
+    double *s_far = s_leg + NL * 3;                                     // Far<N>::kCoef
+    double *s_warp = s_far + Far<N>::kCoef;
     s_warp += (s_warp - s_pv) & 1;                                     // 16-byte aligned
     double *s_wP = s_warp;                                              // 8 x kMaxLQ, until the operands are loaded
     double *s_g = s_warp + warp * warp_doubles<N, PANELS>(LQ);
@@ -150,7 +150,7 @@ __global__ void __launch_bounds__(kWarps * 32, 4) assemble64_kernel(AsmArgs a) {
         }
         s_row[tid] = r;
     }
-    for (int t = tid; t < kFarCoef; t += kWarps * 32) s_far[t] = far_coef(t);
+    for (int t = tid; t < Far<N>::kCoef; t += kWarps * 32) s_far[t] = Far<N>::coef(t);
     if (tid < NL * 3) {
         const int m = tid / 3, p = m - 2 * (tid % 3);
         s_leg[tid] = p >= 0 ? leg_scale(m) * leg_coef(m, p) : 0.0;
@@ -370,7 +370,7 @@ __global__ void __launch_bounds__(kWarps * 32, 4) assemble64_kernel(AsmArgs a) {
 
 template <int N, bool PANELS, int KSMAX, int LQC>
 cudaError_t launch_n(const AsmArgs &a, int nchunks, cudaStream_t st) {
-    const size_t smem = sizeof(double) * (kMaxLQ + 3 * (N + 1) + kFarCoef + 1 +
+    const size_t smem = sizeof(double) * (kMaxLQ + 3 * (N + 1) + Far<N>::kCoef + 1 +
                                           kWarps * (size_t)warp_doubles<N, PANELS>(a.LQ)) +
                         sizeof(RowTab) * (N + 3);
     auto kern = assemble64_kernel<N, PANELS, KSMAX, LQC>;
@@ -393,21 +393,7 @@ cudaError_t launch_ks(const AsmArgs &a, int nchunks, cudaStream_t st) {
 bool assemble64_supported(int N) { return N >= 1 && N <= 5; }
 
 int assemble64_chunks(int M, int sm_count) {
-    // sources per CTA such that rounds of resident CTAs x (sources + the set-up
-    // of a CTA, about one source's time) is smallest; ties: fewer chunks
-    const int64_t ctas = (M + kWarps * kTI - 1) / (kWarps * kTI), slots = 4 * (int64_t)sm_count;
-    int64_t best = -1;
-    int chunks = 1;
-    for (int per = M; per >= 1; --per) {
-        const int c = (M + per - 1) / per;
-        if ((M + c - 1) / c != per) continue;
-        const int64_t cost = ((ctas * c + slots - 1) / slots) * (per + 1);
-        if (best < 0 || cost < best) {
-            best = cost;
-            chunks = c;
-        }
-    }
-    return chunks;
+    return pick_chunks(M, (M + kWarps * kTI - 1) / (kWarps * kTI), 4 * (int64_t)sm_count, 1);
 }
 
 cudaError_t launch_assemble64(const AsmArgs &a, int nchunks, cudaStream_t st) {

@@ -227,13 +227,17 @@ __device__ __forceinline__ int far_top(float c) {
 
 // Step n: I_n = -(1 + r/2) (b/c) I_{n+1} - (1 + r) (1/c) I_{n+2} + r w, r =
 // 1/(n+1), w = (ue -+ ub)/c.  r comes from a table in shared memory for the
-// steps above kFarTail, which run as a loop (a fully unrolled recursion
-// exceeds the instruction cache that a scheduler's warps share).
-constexpr int kFarTail = 8;
-constexpr int kFarTop = 30;
-constexpr int kFarCoef = kFarTop - kFarTail;
-// entry t of the table: r of step kFarTail + 1 + t
-__device__ __forceinline__ double far_coef(int t) { return 1.0 / (kFarTail + 2.0 + t); }
+// steps above Far<N>::kTail, which run as a loop (a fully unrolled recursion
+// exceeds the instruction cache that a scheduler's warps share).  N > 5 needs
+// n up to 10 and starts four steps higher.
+template <int N>
+struct Far {
+    static constexpr int kShift = N <= 5 ? 0 : 4;
+    static constexpr int kTail = N <= 5 ? 8 : 10;
+    static constexpr int kCoef = 30 + kShift - kTail;  // entries of the table
+    // entry t of the table: r of step kTail + 1 + t
+    __device__ __forceinline__ static double coef(int t) { return 1.0 / (kTail + 2.0 + t); }
+};
 
 struct FarState {
     double nicb, hicb, nic, wp, wm, ic;      // -b/c, -b/(2c), -1/c, (ue - ub)/c, (ue + ub)/c, 1/c
@@ -248,7 +252,7 @@ struct FarState {
 
 // the last steps, n .. 0; u_n and v_n to out as soon as they are formed
 template <int N, int n, typename OUT>
-__device__ __forceinline__ void far_tail(FarState &f, double e2, double e6, const OUT &out) {
+__device__ __forceinline__ void far_tail(FarState &f, double e2, double e6, OUT &&out) {
     if constexpr (n >= 0) {
         f.step(1.0 / (n + 1.0), n % 2 == 1 ? f.wp : f.wm);
         if constexpr (n <= N) out.u(n, fma(e2, f.j1, f.i1));
@@ -262,7 +266,7 @@ __device__ __forceinline__ void far_tail(FarState &f, double e2, double e6, cons
 // ue ub = sqrt((1 + c)^2 - b^2) and (ue + ub)^2 = 2 (1 + c + ue ub); ue - ub =
 // 2b / (ue + ub).
 template <int N, typename OUT>
-__device__ __forceinline__ void moments_far_fp64(double b, double c, double eps2, const double *coef, const OUT &out) {
+__device__ __forceinline__ void moments_far_fp64(double b, double c, double eps2, const double *coef, OUT &&out) {
     const double t = 1.0 + c, pp = fma(t, t, -b * b);
     const double us2 = 2.0 * fma(pp, rsqrt_pos(pp), t);
     const double ius = rsqrt_pos(us2);
@@ -274,19 +278,19 @@ __device__ __forceinline__ void moments_far_fp64(double b, double c, double eps2
     f.wp = -2.0 * f.nicb * ius;
     f.wm = us2 * ius * f.ic;
     f.i1 = f.i2 = f.j1 = f.j2 = f.s1 = f.s2 = 0.0;
-    const double *k = coef + (far_top((float)c) - kFarTail - 2);  // of the odd step below the start
+    const double *k = coef + (far_top((float)c) + Far<N>::kShift - Far<N>::kTail - 2);  // of the odd step below the start
 #pragma unroll 1
     for (; k >= coef; k -= 2) {
         f.step(k[1], f.wm);  // even n
         f.step(k[0], f.wp);  // odd n
     }
     const double e2 = 2.0 * eps2 * f.ic;
-    far_tail<N, kFarTail>(f, e2, -3.0 * e2 * f.ic, out);
+    far_tail<N, Far<N>::kTail>(f, e2, -3.0 * e2 * f.ic, out);
 }
 
 // The same families of any point from the reference's moments.
 template <int N, typename OUT>
-__device__ __forceinline__ void moments_near_uv(double b, double c, double eps2, const OUT &out) {
+__device__ __forceinline__ void moments_near_uv(double b, double c, double eps2, OUT &&out) {
     double I[N + 3], J[N + 3], S[N + 3];
     moments_fp64<N>(b, c, I, J, S);
 #pragma unroll

@@ -69,6 +69,24 @@ inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
+// Source chunks of a grid of ctas x chunks CTAs, slots of them resident: the
+// share of sources per CTA for which rounds x (share + setup) is smallest,
+// setup = a CTA's set-up in units of one source's time; ties: the larger share.
+inline int pick_chunks(int M, int64_t ctas, int64_t slots, int setup) {
+    int64_t best = -1;
+    int chunks = 1;
+    for (int share = M; share >= 1; --share) {
+        const int c = (M + share - 1) / share;
+        if ((M + c - 1) / c != share) continue;  // the same chunks with a smaller share
+        const int64_t cost = ((ctas * c + slots - 1) / slots) * (share + setup);
+        if (best < 0 || cost < best) {
+            best = cost;
+            chunks = c;
+        }
+    }
+    return chunks;
+}
+
 struct AsmArgs {
     int M, N, LQ;
     int t0, t1;                // target fibers [t0, t1) (a row-block shard; 0, M for the whole system)
@@ -151,8 +169,9 @@ struct VelArgs {
     int chunk;
 };
 cudaError_t launch_velocity(const VelArgs &a, bool numeric, int nchunks, cudaStream_t st);
+int pair_sum_chunks(int M, int sm_count);  // source chunks of launch_velocity and launch_matfree
 
-// Matrix-free FP64 product y = A x (matfree.cu), the reference's mat_prod.
+// Matrix-free FP64 product y = A x (pair_sum.cu), the reference's mat_prod.
 struct MatfreeArgs {
     int M, N, LQ;
     int64_t n;                 // 3 N M
