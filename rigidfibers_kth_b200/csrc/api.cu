@@ -1,8 +1,6 @@
 // api.cu - the C ABI (include/rigidfibers.h): handle life cycle and the
 // reference step API (src/simulation.cu:40-424 of the reference):
 // assemble_system -> solve_system -> update_velocities -> update_fibers.
-#include <cublas_v2.h>
-
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
@@ -47,13 +45,12 @@ void free_all(rf_handle *h) {
         cudaFree(h->V[i]);
         cudaFree(h->W[i]);
     }
-    void *ptrs[] = {h->tab, h->A64, h->LU, h->lu_r, h->lu_piv, h->lu_info, h->mfpart, h->A32, h->A16, h->b, h->x, h->bpart, h->velpart, h->PV64, h->PW64,
+    void *ptrs[] = {h->tab, h->A64, h->LU, h->lu_r, h->lu_piv, h->lu_info, h->mfpart, h->mvx, h->A32, h->A16, h->b, h->x, h->bpart, h->velpart, h->PV64, h->PW64,
                     h->PV32, h->PW32, h->vpart, h->pvx, h->pwx, h->work64, h->work32, h->r64, h->r32,
                     h->d32, h->x32, h->Pblocks, h->knn, h->mlp_w, h->mlp_wtc, h->mlp_err, h->feat, h->mlp_h1, h->mlp_h2, h->mlp_out,
                     h->dscal, h->rb.partials, h->rb.counter, h->near_bits, h->near_list, h->near_cnt,
                     h->far_contr, h->near_contr, h->near_pref, h->near_off, h->near_total, h->nearbuf};
     for (void *p : ptrs) cudaFree(p);
-    if (h->blas) cublasDestroy(static_cast<cublasHandle_t>(h->blas));
     h->gm64.reset();
     h->gm32.reset();
     if (h->hscal) cudaFreeHost(h->hscal);
@@ -191,6 +188,13 @@ constexpr int kPcRetry = 8;
 constexpr double kPcDamping = 0.85;
 constexpr int kPcExplore = 32;
 
+
+// Device copies of the operand and the result of rf_matvec and
+// rf_matvec_free, kept by the handle: an allocation and a release per call cost
+// up to 0.8 ms where the driver maps and unmaps a block of its own for them.
+cudaError_t product_buffers(rf_handle *h) {
+    return h->mvx ? cudaSuccess : dalloc(&h->mvx, 2 * (size_t)h->n);
+}
 
 // Sum the recorded start/stop pairs of the product timer (waits for them).
 cudaError_t gemv_timer_flush(rf_handle *h) {
@@ -750,24 +754,20 @@ rf_status rf_solve_system(rf_handle *h) {
         // dgesv (coeffs_and_vels.f90:62,158): LU factors of a copy of A (A
         // itself stays available to rf_get_matrix and rf_matvec), then the two
         // triangular solves; the factors' buffer is made at the first call
-        const size_t mat = sizeof(double) * (size_t)h->lda * (size_t)h->n;
+        const size_t mat = (size_t)h->lda * (size_t)h->n;
         if (!h->LU) {
-            CK(h, cudaMalloc(&h->LU, mat), "direct solver: LU factors (one more n x n FP64 matrix)");
+            CK(h, dalloc(&h->LU, mat + h->lda), "direct solver: LU factors (one more n x n FP64 matrix)");
             CK(h, cudaMalloc(&h->lu_r, sizeof(double) * h->n), "direct solver");
             CK(h, cudaMalloc(&h->lu_piv, sizeof(int) * h->n), "direct solver");
             CK(h, cudaMalloc(&h->lu_info, sizeof(int)), "direct solver");
         }
-        if (!h->blas) {
-            cublasHandle_t bh = nullptr;
-            if (cublasCreate(&bh) != CUBLAS_STATUS_SUCCESS)
-                return rf::fail(h, RF_ERR_CUDA, "direct solver: cuBLAS handle could not be created");
-            h->blas = bh;
-        }
-        CK(h, cudaMemcpyAsync(h->LU, h->A64, mat, cudaMemcpyDeviceToDevice, st), "direct solver");
-        CK(h, cudaMemcpyAsync(h->x, h->b, sizeof(double) * h->n, cudaMemcpyDeviceToDevice, st), "direct solver");
-        CK(h, rf::lu_factor(h->LU, h->lda, h->n, h->lu_piv, h->lu_info, h->blas, st, &h->launches),
+        double *y = h->LU + mat;  // the right-hand side as a last column
+        CK(h, cudaMemcpyAsync(h->LU, h->A64, sizeof(double) * mat, cudaMemcpyDeviceToDevice, st), "direct solver");
+        CK(h, cudaMemcpyAsync(y, h->b, sizeof(double) * h->n, cudaMemcpyDeviceToDevice, st), "direct solver");
+        CK(h, rf::lu_factor(h->LU, h->lda, h->n, h->n + 1, h->lu_piv, h->lu_info, st, &h->launches),
            "LU factorisation");
-        CK(h, rf::lu_solve(h->LU, h->lda, h->n, h->lu_piv, h->x, st, &h->launches), "LU solve");
+        CK(h, rf::lu_back(h->LU, h->lda, h->n, y, st, &h->launches), "LU solve");
+        CK(h, cudaMemcpyAsync(h->x, y, sizeof(double) * h->n, cudaMemcpyDeviceToDevice, st), "direct solver");
         // backward error |b - A x| / |b| for the statistics
         CK(h, (rf::launch_gemv<double, double, double, double>(h->A64, h->lda, h->n, h->n, h->x, h->lu_r, h->b,
                                                                 h->work64, h->work_elems, h->sm_count, st)),
@@ -1250,10 +1250,9 @@ rf_status rf_matvec(rf_handle *h, const double *x, double *y) {
     if (!h || !x || !y) return rf::fail(h, RF_ERR_INVALID_ARG, "null argument");
     if (h->shards > 1) return rf::fail(h, RF_ERR_INVALID_ARG, "rf_matvec needs the whole system (not a row-block shard)");
     CK(h, cudaSetDevice(h->device), "cudaSetDevice");
-    double *dx = nullptr, *dy = nullptr;
-    CK(h, cudaMalloc(&dx, h->n * 8), "alloc");
-    cudaError_t e = cudaMalloc(&dy, h->n * 8);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(dx, x, h->n * 8, cudaMemcpyHostToDevice, h->stream);
+    CK(h, product_buffers(h), "alloc");
+    double *dx = h->mvx, *dy = h->mvx + h->n;
+    cudaError_t e = cudaMemcpyAsync(dx, x, h->n * 8, cudaMemcpyHostToDevice, h->stream);
     if (e == cudaSuccess) {
         if (h->A64)
             e = rf::launch_gemv<double, double, double, double>(h->A64, h->lda, h->n, h->n, dx, dy, nullptr, h->work64,
@@ -1269,8 +1268,6 @@ rf_status rf_matvec(rf_handle *h, const double *x, double *y) {
     }
     if (e == cudaSuccess) e = cudaMemcpyAsync(y, dy, h->n * 8, cudaMemcpyDeviceToHost, h->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-    cudaFree(dx);
-    cudaFree(dy);
     CK(h, e, "matvec");
     return RF_OK;
 }
@@ -1288,16 +1285,13 @@ rf_status rf_dgesv(int64_t n, const double *A, int64_t lda, const double *b, dou
     struct Scope {
         int prev;
         cudaStream_t st = nullptr;
-        cublasHandle_t blas = nullptr;
-        double *dA = nullptr, *dx = nullptr;
+        double *dA = nullptr;
         int *dpiv = nullptr, *dinfo = nullptr;
         ~Scope() {
             if (st) cudaStreamSynchronize(st);
             cudaFree(dA);
-            cudaFree(dx);
             cudaFree(dpiv);
             cudaFree(dinfo);
-            if (blas) cublasDestroy(blas);
             if (st) cudaStreamDestroy(st);
             cudaSetDevice(prev);
         }
@@ -1310,19 +1304,19 @@ rf_status rf_dgesv(int64_t n, const double *A, int64_t lda, const double *b, dou
     cudaError_t e = cudaStreamCreateWithFlags(&sc.st, cudaStreamNonBlocking);
     if (e != cudaSuccess) return cuda(e, "stream");
     const size_t nn = (size_t)n;
-    if ((e = cudaMalloc(&sc.dA, sizeof(double) * nn * nn)) != cudaSuccess) return cuda(e, "device copy of A");
-    if ((e = cudaMalloc(&sc.dx, sizeof(double) * nn)) != cudaSuccess ||
-        (e = cudaMalloc(&sc.dpiv, sizeof(int) * nn)) != cudaSuccess ||
+    // the matrix, then the right-hand side as a last column
+    const size_t ld = (size_t)round_up(n, 16);
+    if ((e = dalloc(&sc.dA, ld * (nn + 1))) != cudaSuccess) return cuda(e, "device copy of A");
+    if ((e = cudaMalloc(&sc.dpiv, sizeof(int) * nn)) != cudaSuccess ||
         (e = cudaMalloc(&sc.dinfo, sizeof(int))) != cudaSuccess)
         return cuda(e, "device buffers");
-    if (cublasCreate(&sc.blas) != CUBLAS_STATUS_SUCCESS)
-        return rf::fail(nullptr, RF_ERR_CUDA, "rf_dgesv: cuBLAS handle could not be created");
-    if ((e = cudaMemcpy2DAsync(sc.dA, sizeof(double) * nn, A, sizeof(double) * (size_t)lda, sizeof(double) * nn, nn,
+    double *dx = sc.dA + ld * nn;
+    if ((e = cudaMemcpy2DAsync(sc.dA, sizeof(double) * ld, A, sizeof(double) * (size_t)lda, sizeof(double) * nn, nn,
                                cudaMemcpyHostToDevice, sc.st)) != cudaSuccess ||
-        (e = cudaMemcpyAsync(sc.dx, b, sizeof(double) * nn, cudaMemcpyHostToDevice, sc.st)) != cudaSuccess)
+        (e = cudaMemcpyAsync(dx, b, sizeof(double) * nn, cudaMemcpyHostToDevice, sc.st)) != cudaSuccess)
         return cuda(e, "upload");
     int64_t launches = 0;
-    if ((e = rf::lu_factor(sc.dA, n, n, sc.dpiv, sc.dinfo, sc.blas, sc.st, &launches)) != cudaSuccess)
+    if ((e = rf::lu_factor(sc.dA, ld, n, n + 1, sc.dpiv, sc.dinfo, sc.st, &launches)) != cudaSuccess)
         return cuda(e, "LU factorisation");
     int hinfo = 0;
     if ((e = cudaMemcpyAsync(&hinfo, sc.dinfo, sizeof(int), cudaMemcpyDeviceToHost, sc.st)) != cudaSuccess ||
@@ -1330,9 +1324,9 @@ rf_status rf_dgesv(int64_t n, const double *A, int64_t lda, const double *b, dou
         return cuda(e, "LU factorisation");
     *info = hinfo;
     if (hinfo == 0) {
-        if ((e = rf::lu_solve(sc.dA, n, n, sc.dpiv, sc.dx, sc.st, &launches)) != cudaSuccess)
+        if ((e = rf::lu_back(sc.dA, ld, n, dx, sc.st, &launches)) != cudaSuccess)
             return cuda(e, "LU solve");
-        if ((e = cudaMemcpyAsync(x, sc.dx, sizeof(double) * nn, cudaMemcpyDeviceToHost, sc.st)) != cudaSuccess)
+        if ((e = cudaMemcpyAsync(x, dx, sizeof(double) * nn, cudaMemcpyDeviceToHost, sc.st)) != cudaSuccess)
             return cuda(e, "download");
     }
     if (ipiv) {
@@ -1349,12 +1343,18 @@ rf_status rf_dgesv(int64_t n, const double *A, int64_t lda, const double *b, dou
 rf_status rf_matvec_free(rf_handle *h, const double *x, double *y) {
     if (!h || !x || !y) return rf::fail(h, RF_ERR_INVALID_ARG, "null argument");
     CK(h, cudaSetDevice(h->device), "cudaSetDevice");
-    if (!h->mfpart)
-        CK(h, cudaMalloc(&h->mfpart, sizeof(double) * (size_t)h->vel_chunks * h->n), "matrix-free product partials");
-    double *dx = nullptr, *dy = nullptr;
-    CK(h, cudaMalloc(&dx, h->n * 8), "alloc");
-    cudaError_t e = cudaMalloc(&dy, h->n * 8);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(dx, x, h->n * 8, cudaMemcpyHostToDevice, h->stream);
+    // partials, operand and result in the stored products' workspace where it
+    // holds them (nearly always), else in buffers made at the first call
+    const int64_t parts = (int64_t)h->vel_chunks * h->n;
+    double *part = h->work64, *dx = h->work64 + parts;
+    if (parts + 2 * h->n > h->work_elems) {
+        if (!h->mfpart) CK(h, dalloc(&h->mfpart, (size_t)parts), "matrix-free product partials");
+        CK(h, product_buffers(h), "alloc");
+        part = h->mfpart;
+        dx = h->mvx;
+    }
+    double *dy = dx + h->n;
+    cudaError_t e = cudaMemcpyAsync(dx, x, h->n * 8, cudaMemcpyHostToDevice, h->stream);
     if (e == cudaSuccess) {
         rf::MatfreeArgs a{};
         a.M = h->M;
@@ -1365,15 +1365,13 @@ rf_status rf_matvec_free(rf_handle *h, const double *x, double *y) {
         a.ori = h->T[h->cur];
         a.x = dx;
         a.tab = h->tab;
-        a.part = h->mfpart;
+        a.part = part;
         a.chunk = h->vel_chunk;
         e = rf::launch_matfree(a, h->p.use_analytical_integration == 0, h->vel_chunks, dx, dy, h->stream);
         h->launches += 2;
     }
     if (e == cudaSuccess) e = cudaMemcpyAsync(y, dy, h->n * 8, cudaMemcpyDeviceToHost, h->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-    cudaFree(dx);
-    cudaFree(dy);
     CK(h, e, "matrix-free product");
     return RF_OK;
 }

@@ -41,7 +41,6 @@ struct rf_handle {
     double *lu_r = nullptr;    // direct solver: residual b - A x for the statistics
     int *lu_piv = nullptr;     // [n] pivot rows
     int *lu_info = nullptr;
-    void *blas = nullptr;      // direct solver: cuBLAS handle (cublasHandle_t), made at the first direct solve
     float *A32 = nullptr;
     __nv_bfloat16 *A16 = nullptr;   // BF16 matrix; in split storage also the high plane
     unsigned short *A16lo = nullptr;  // split storage (mixed BF16): the low plane, a_plane entries after A16
@@ -53,7 +52,8 @@ struct rf_handle {
     bool asm64 = false;        // FP64 analytic assembly by autonomous warps (assemble64.cu)
     int vel_chunks = 1, vel_chunk = 1;
     double *velpart = nullptr; // [vel_chunks][6M]
-    double *mfpart = nullptr;  // [vel_chunks][n] matrix-free product partials, made at its first use
+    double *mvx = nullptr;     // [2n] operand and result of rf_matvec (and of rf_matvec_free), made at their first use
+    double *mfpart = nullptr;  // [vel_chunks][n] matrix-free product partials where work64 is too small
     // velocity panels (reuse mode)
     double *PV64 = nullptr, *PW64 = nullptr;
     float *PV32 = nullptr, *PW32 = nullptr;

@@ -228,15 +228,15 @@ cudaError_t launch_mgs_norm(int64_t n, T *w, const T *vprev, const double *hprev
 template <typename T>
 cudaError_t launch_dot(int64_t n, const T *a, const T *b, double *out, const RedBuf &rb, cudaStream_t st);
 
-// Direct solve (lu.cu): A (n x n, column-major, ld lda) is overwritten by its
-// LU factors with partial pivoting, piv[n] the pivot rows (0-based), info the
-// first zero pivot (1-based) or 0; lu_solve overwrites x (= b on entry) with
-// the solution.  blas: a cuBLAS handle (the trailing updates); launches counts
-// the kernels launched.
-cudaError_t lu_factor(double *A, int64_t lda, int64_t n, int *piv, int *info, void *blas, cudaStream_t st,
+// Direct solve (lu.cu): the first n columns of A (column-major, even ld lda,
+// 16-byte aligned) are overwritten by their LU factors with partial pivoting
+// (L's rows left of a panel unswapped), the columns n .. ncols - 1 by L^-1 P of
+// themselves (right-hand sides); piv[n] the pivot rows (0-based), info the
+// first zero pivot (1-based) or 0.  lu_back overwrites x (such a column) with
+// U^-1 x.  launches counts the kernels launched.
+cudaError_t lu_factor(double *A, int64_t lda, int64_t n, int64_t ncols, int *piv, int *info, cudaStream_t st,
                       int64_t *launches);
-cudaError_t lu_solve(const double *A, int64_t lda, int64_t n, const int *piv, double *x, cudaStream_t st,
-                     int64_t *launches);
+cudaError_t lu_back(const double *A, int64_t lda, int64_t n, double *x, cudaStream_t st, int64_t *launches);
 // y = alpha_scale * x where alpha_scale = num/den (den device scalar), i.e. y = x * (num / *den)
 template <typename TO, typename TI>
 cudaError_t launch_scale(int64_t n, const TI *x, const double *den, double num, TO *y, cudaStream_t st);
