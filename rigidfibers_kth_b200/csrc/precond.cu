@@ -28,7 +28,7 @@
 //                  rotation- and sign-free part.
 //
 // The MLP (144 -> 256 -> 256 -> 225, ReLU) is trained by the trainer below
-// with hand-written FP32 GEMM kernels (forward and backward) and Adam.
+// with the FP32 kernels of mlp_train.cu (forward, backward, Adam).
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -36,6 +36,7 @@
 #include <vector>
 
 #include "handle.h"
+#include "mlp_train.h"
 
 namespace rf {
 namespace {
@@ -347,149 +348,6 @@ __global__ void pair_frame_kernel(int M, int kp, const float *__restrict__ rot, 
         }
 }
 
-// ------------------------------------------------------------------ FP32 GEMM
-// C[i][j] = act( alpha * sum_k A(i,k) B(k,j) + bias[j] ) (+ beta C), generic
-// strides so one kernel serves X W^T, dY W and dY^T X.  64x64 tiles, 16-deep,
-// 256 threads with 4x4 outputs each.
-struct GemmArgs {
-    int m, n, k;
-    const float *A;
-    int64_t sai, sak;
-    const float *B;
-    int64_t sbk, sbj;
-    float *C;
-    int64_t ldc;
-    const float *bias;
-    int relu;
-    float beta;
-};
-
-__global__ void __launch_bounds__(256) gemm_kernel(GemmArgs g) {
-    __shared__ float As[16][64 + 4];
-    __shared__ float Bs[16][64 + 4];
-    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-    const int i0 = blockIdx.y * 64, j0 = blockIdx.x * 64;
-    float acc[4][4] = {};
-    for (int k0 = 0; k0 < g.k; k0 += 16) {
-        for (int t = threadIdx.x; t < 16 * 64; t += 256) {
-            const int kk = t / 64, r = t % 64;
-            const int gi = i0 + r, gk = k0 + kk;
-            As[kk][r] = (gi < g.m && gk < g.k) ? g.A[gi * g.sai + gk * g.sak] : 0.f;
-            const int gj = j0 + r;
-            Bs[kk][r] = (gj < g.n && gk < g.k) ? g.B[gk * g.sbk + gj * g.sbj] : 0.f;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int kk = 0; kk < 16; ++kk) {
-            float a[4], b[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                a[u] = As[kk][ty * 4 + u];
-                b[u] = Bs[kk][tx * 4 + u];
-            }
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-#pragma unroll
-                for (int v = 0; v < 4; ++v) acc[u][v] += a[u] * b[v];
-        }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int u = 0; u < 4; ++u)
-#pragma unroll
-        for (int v = 0; v < 4; ++v) {
-            const int i = i0 + ty * 4 + u, j = j0 + tx * 4 + v;
-            if (i >= g.m || j >= g.n) continue;
-            float val = acc[u][v];
-            if (g.bias) val += g.bias[j];
-            if (g.relu) val = fmaxf(val, 0.f);
-            float *c = g.C + (int64_t)i * g.ldc + j;
-            *c = g.beta != 0.f ? g.beta * *c + val : val;
-        }
-}
-
-cudaError_t gemm(const GemmArgs &g, cudaStream_t st) {
-    dim3 grid((g.n + 63) / 64, (g.m + 63) / 64);
-    gemm_kernel<<<grid, 256, 0, st>>>(g);
-    return cudaGetLastError();
-}
-
-// column sums of an m x n row-major matrix (bias gradients)
-__global__ void colsum_kernel(int m, int n, const float *__restrict__ X, float *__restrict__ out) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n) return;
-    float s = 0.f;
-    for (int i = 0; i < m; ++i) s += X[(int64_t)i * n + j];
-    out[j] = s;
-}
-
-// dY = 2 (Y - T) / count, and per-block partial sums of (Y - T)^2
-__global__ void mse_grad_kernel(int64_t cnt, const float *__restrict__ Y, const float *__restrict__ T,
-                                float *__restrict__ dY, double *__restrict__ part) {
-    __shared__ double sh[256];
-    double acc = 0.0;
-    for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < cnt; e += (int64_t)gridDim.x * blockDim.x) {
-        const float d = Y[e] - T[e];
-        dY[e] = 2.f * d / (float)cnt;
-        acc += (double)d * d;
-    }
-    sh[threadIdx.x] = acc;
-    __syncthreads();
-    for (int o = 128; o > 0; o >>= 1) {
-        if (threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) part[blockIdx.x] = sh[0];
-}
-
-__global__ void relu_back_kernel(int64_t cnt, const float *__restrict__ H, float *__restrict__ dH) {
-    for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < cnt; e += (int64_t)gridDim.x * blockDim.x)
-        if (H[e] <= 0.f) dH[e] = 0.f;
-}
-
-__global__ void adam_kernel(int64_t cnt, float *__restrict__ w, const float *__restrict__ g, float *__restrict__ m,
-                            float *__restrict__ v, float lr, float b1, float b2, float c1, float c2, float eps) {
-    for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < cnt; e += (int64_t)gridDim.x * blockDim.x) {
-        const float gi = g[e];
-        const float mi = b1 * m[e] + (1.f - b1) * gi;
-        const float vi = b2 * v[e] + (1.f - b2) * gi * gi;
-        m[e] = mi;
-        v[e] = vi;
-        w[e] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
-    }
-}
-
-__global__ void gather_rows_kernel(int rows, int width, const int *__restrict__ idx, const float *__restrict__ src,
-                                   float *__restrict__ dst) {
-    const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= (int64_t)rows * width) return;
-    const int r = (int)(e / width), c = (int)(e - (int64_t)r * width);
-    dst[e] = src[(int64_t)idx[r] * width + c];
-}
-
-// parameter offsets inside the packed weight vector
-struct MlpLayout {
-    int64_t w1 = 0, b1 = w1 + (int64_t)kHid * kIn, w2 = b1 + kHid, b2 = w2 + (int64_t)kHid * kHid, w3 = b2 + kHid,
-            b3 = w3 + (int64_t)kOut * kHid, total = b3 + kOut;
-};
-
-// Forward pass for `rows` samples: H1, H2, O (row-major)
-cudaError_t mlp_forward(const float *W, int rows, const float *X, float *H1, float *H2, float *O, cudaStream_t st) {
-    const MlpLayout L;
-    GemmArgs g{};
-    g.m = rows; g.n = kHid; g.k = kIn;
-    g.A = X; g.sai = kIn; g.sak = 1;
-    g.B = W + L.w1; g.sbk = 1; g.sbj = kIn;           // B(k,j) = W1[j][k]
-    g.C = H1; g.ldc = kHid; g.bias = W + L.b1; g.relu = 1;
-    cudaError_t e = gemm(g, st);
-    if (e != cudaSuccess) return e;
-    g.k = kHid; g.A = H1; g.sai = kHid; g.B = W + L.w2; g.sbj = kHid; g.C = H2; g.bias = W + L.b2;
-    e = gemm(g, st);
-    if (e != cudaSuccess) return e;
-    g.n = kOut; g.A = H2; g.B = W + L.w3; g.sbj = kHid; g.C = O; g.ldc = kOut; g.bias = W + L.b3; g.relu = 0;
-    return gemm(g, st);
-}
-
 }  // namespace
 
 // ------------------------------------------------------------------ handle side
@@ -643,11 +501,12 @@ struct rf_trainer {
     float *W = nullptr, *G = nullptr, *Mom = nullptr, *Var = nullptr;
     float *X = nullptr, *Y = nullptr;      // dataset
     int64_t count = 0, cap = 0;
-    float *bx = nullptr, *by = nullptr, *h1 = nullptr, *h2 = nullptr, *o = nullptr, *dO = nullptr, *dh2 = nullptr,
-          *dh1 = nullptr;
-    int *bidx = nullptr;
+    float *bx = nullptr, *by = nullptr;    // a batch
+    rf::MlpBatch b{};                      // and its intermediate results
     int bcap = 0;
-    double *part = nullptr;
+    int *perm = nullptr;                   // an epoch's order of the samples
+    int64_t perm_cap = 0;
+    double *sse = nullptr;                 // summed squared error
     int64_t t = 0;
     std::mt19937_64 rng;
 };
@@ -784,7 +643,8 @@ rf_status rf_trainer_create(int32_t device, uint64_t seed, rf_trainer **out) {
     bool ok = cudaStreamCreateWithFlags(&t->stream, cudaStreamNonBlocking) == cudaSuccess &&
               cudaMalloc(&t->W, sizeof(float) * P) == cudaSuccess && cudaMalloc(&t->G, sizeof(float) * P) == cudaSuccess &&
               cudaMalloc(&t->Mom, sizeof(float) * P) == cudaSuccess && cudaMalloc(&t->Var, sizeof(float) * P) == cudaSuccess &&
-              cudaMalloc(&t->part, sizeof(double) * 1024) == cudaSuccess;
+              cudaMalloc(&t->b.part, sizeof(float) * P * kMlpSlices) == cudaSuccess &&
+              cudaMalloc(&t->sse, sizeof(double)) == cudaSuccess;
     if (!ok) {
         rf_trainer_destroy(t);
         return fail(nullptr, RF_ERR_OOM, "trainer allocation");
@@ -810,8 +670,8 @@ rf_status rf_trainer_create(int32_t device, uint64_t seed, rf_trainer **out) {
 rf_status rf_trainer_destroy(rf_trainer *t) {
     if (!t) return RF_ERR_INVALID_ARG;
     cudaSetDevice(t->device);
-    void *ptrs[] = {t->W, t->G, t->Mom, t->Var, t->X, t->Y, t->bx, t->by, t->h1, t->h2, t->o, t->dO, t->dh2, t->dh1,
-                    t->bidx, t->part};
+    void *ptrs[] = {t->W, t->G, t->Mom, t->Var, t->X, t->Y, t->bx, t->by, t->b.h1, t->b.h2, t->b.dO, t->b.dh2,
+                    t->b.dh1, t->b.part, t->b.sse, t->perm, t->sse};
     for (void *p : ptrs) cudaFree(p);
     if (t->stream) cudaStreamDestroy(t->stream);
     delete t;
@@ -849,77 +709,20 @@ rf_status rf_trainer_add_samples(rf_trainer *t, const float *features, const flo
 namespace {
 bool ensure_batch(rf_trainer *t, int B) {
     if (B <= t->bcap) return true;
-    void *ptrs[] = {t->bx, t->by, t->h1, t->h2, t->o, t->dO, t->dh2, t->dh1, t->bidx};
+    void *ptrs[] = {t->bx, t->by, t->b.h1, t->b.h2, t->b.dO, t->b.dh2, t->b.dh1, t->b.sse};
     for (void *p : ptrs) cudaFree(p);
-    bool ok = cudaMalloc(&t->bx, sizeof(float) * B * kIn) == cudaSuccess &&
-              cudaMalloc(&t->by, sizeof(float) * B * kOut) == cudaSuccess &&
-              cudaMalloc(&t->h1, sizeof(float) * B * kHid) == cudaSuccess &&
-              cudaMalloc(&t->h2, sizeof(float) * B * kHid) == cudaSuccess &&
-              cudaMalloc(&t->o, sizeof(float) * B * kOut) == cudaSuccess &&
-              cudaMalloc(&t->dO, sizeof(float) * B * kOut) == cudaSuccess &&
-              cudaMalloc(&t->dh2, sizeof(float) * B * kHid) == cudaSuccess &&
-              cudaMalloc(&t->dh1, sizeof(float) * B * kHid) == cudaSuccess &&
-              cudaMalloc(&t->bidx, sizeof(int) * B) == cudaSuccess;
+    auto f = [](float **p, int64_t n) {
+        *p = nullptr;
+        return cudaMalloc(p, sizeof(float) * n) == cudaSuccess;
+    };
+    t->b.sse = nullptr;
+    const int64_t n = B;
+    const bool ok = f(&t->bx, n * kIn) & f(&t->by, n * kOut) & f(&t->b.h1, n * kHid) & f(&t->b.h2, n * kHid) &
+                    f(&t->b.dO, n * kMlpOutLd) & f(&t->b.dh2, n * kHid) & f(&t->b.dh1, n * kHid) &
+                    (cudaMalloc(&t->b.sse, sizeof(double) * mlp_loss_parts(B)) == cudaSuccess);
+    if (!ok) cudaGetLastError();
     t->bcap = ok ? B : 0;
     return ok;
-}
-
-// forward + backward on B samples already in bx/by; gradient into G; returns
-// the summed squared error (over B*225 outputs)
-cudaError_t forward_backward(rf_trainer *t, int B, double *sse) {
-    const MlpLayout L;
-    cudaStream_t st = t->stream;
-    cudaError_t e = mlp_forward(t->W, B, t->bx, t->h1, t->h2, t->o, st);
-    if (e != cudaSuccess) return e;
-    const int64_t cnt = (int64_t)B * kOut;
-    const int nblk = (int)std::min<int64_t>(1024, (cnt + 255) / 256);
-    mse_grad_kernel<<<nblk, 256, 0, st>>>(cnt, t->o, t->by, t->dO, t->part);
-    // layer 3: dW3 = dO^T H2, db3 = colsum dO, dH2 = dO W3 (relu mask)
-    GemmArgs g{};
-    g.m = kOut; g.n = kHid; g.k = B;
-    g.A = t->dO; g.sai = 1; g.sak = kOut;           // A(i,k) = dO[k][i]
-    g.B = t->h2; g.sbk = kHid; g.sbj = 1;
-    g.C = t->G + L.w3; g.ldc = kHid;
-    if ((e = gemm(g, st)) != cudaSuccess) return e;
-    colsum_kernel<<<(kOut + 255) / 256, 256, 0, st>>>(B, kOut, t->dO, t->G + L.b3);
-    g = GemmArgs{};
-    g.m = B; g.n = kHid; g.k = kOut;
-    g.A = t->dO; g.sai = kOut; g.sak = 1;
-    g.B = t->W + L.w3; g.sbk = kHid; g.sbj = 1;     // B(k,j) = W3[k][j]
-    g.C = t->dh2; g.ldc = kHid;
-    if ((e = gemm(g, st)) != cudaSuccess) return e;
-    relu_back_kernel<<<256, 256, 0, st>>>((int64_t)B * kHid, t->h2, t->dh2);
-    // layer 2
-    g = GemmArgs{};
-    g.m = kHid; g.n = kHid; g.k = B;
-    g.A = t->dh2; g.sai = 1; g.sak = kHid;
-    g.B = t->h1; g.sbk = kHid; g.sbj = 1;
-    g.C = t->G + L.w2; g.ldc = kHid;
-    if ((e = gemm(g, st)) != cudaSuccess) return e;
-    colsum_kernel<<<1, 256, 0, st>>>(B, kHid, t->dh2, t->G + L.b2);
-    g = GemmArgs{};
-    g.m = B; g.n = kHid; g.k = kHid;
-    g.A = t->dh2; g.sai = kHid; g.sak = 1;
-    g.B = t->W + L.w2; g.sbk = kHid; g.sbj = 1;
-    g.C = t->dh1; g.ldc = kHid;
-    if ((e = gemm(g, st)) != cudaSuccess) return e;
-    relu_back_kernel<<<256, 256, 0, st>>>((int64_t)B * kHid, t->h1, t->dh1);
-    // layer 1
-    g = GemmArgs{};
-    g.m = kHid; g.n = kIn; g.k = B;
-    g.A = t->dh1; g.sai = 1; g.sak = kHid;
-    g.B = t->bx; g.sbk = kIn; g.sbj = 1;
-    g.C = t->G + L.w1; g.ldc = kIn;
-    if ((e = gemm(g, st)) != cudaSuccess) return e;
-    colsum_kernel<<<1, 256, 0, st>>>(B, kHid, t->dh1, t->G + L.b1);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    std::vector<double> part(nblk);
-    e = cudaMemcpyAsync(part.data(), t->part, sizeof(double) * nblk, cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    double s = 0.0;
-    for (double v : part) s += v;
-    *sse = s;
-    return e;
 }
 }  // namespace
 
@@ -927,33 +730,39 @@ rf_status rf_trainer_train(rf_trainer *t, int32_t epochs, int32_t batch, float l
     if (!t || epochs < 1 || batch < 1 || t->count < 1) return fail(nullptr, RF_ERR_INVALID_ARG, "bad training call");
     cudaSetDevice(t->device);
     if (!ensure_batch(t, batch)) return fail(nullptr, RF_ERR_OOM, "batch buffers");
-    const int64_t P = MlpLayout().total;
+    if (t->count > t->perm_cap) {
+        cudaFree(t->perm);
+        t->perm = nullptr;
+        t->perm_cap = 0;
+        if (cudaMalloc(&t->perm, sizeof(int) * t->count) != cudaSuccess) {
+            cudaGetLastError();
+            return fail(nullptr, RF_ERR_OOM, "sample order");
+        }
+        t->perm_cap = t->count;
+    }
+    // An epoch is queued without waiting for the device: the order of the
+    // samples goes up once, the squared error is summed on the device.
     std::vector<int> perm(t->count);
-    double last = 0.0;
+    double sse = 0.0;
     for (int ep = 0; ep < epochs; ++ep) {
         for (int64_t i = 0; i < t->count; ++i) perm[i] = (int)i;
         std::shuffle(perm.begin(), perm.end(), t->rng);
-        double sse = 0.0;
-        for (int64_t b0 = 0; b0 < t->count; b0 += batch) {
+        cudaError_t e = cudaMemcpyAsync(t->perm, perm.data(), sizeof(int) * t->count, cudaMemcpyHostToDevice, t->stream);
+        if (e == cudaSuccess) e = cudaMemsetAsync(t->sse, 0, sizeof(double), t->stream);
+        for (int64_t b0 = 0; b0 < t->count && e == cudaSuccess; b0 += batch) {
             const int B = (int)std::min<int64_t>(batch, t->count - b0);
-            cudaMemcpyAsync(t->bidx, perm.data() + b0, sizeof(int) * B, cudaMemcpyHostToDevice, t->stream);
-            gather_rows_kernel<<<(unsigned)(((int64_t)B * kIn + 255) / 256), 256, 0, t->stream>>>(B, kIn, t->bidx, t->X,
-                                                                                                  t->bx);
-            gather_rows_kernel<<<(unsigned)(((int64_t)B * kOut + 255) / 256), 256, 0, t->stream>>>(B, kOut, t->bidx,
-                                                                                                   t->Y, t->by);
-            double s = 0.0;
-            cudaError_t e = forward_backward(t, B, &s);
-            if (e != cudaSuccess) return cuda_fail(nullptr, e, "training step");
-            sse += s;
+            e = mlp_gather(B, t->perm + b0, t->X, t->Y, t->bx, t->by, t->stream);
+            if (e == cudaSuccess) e = mlp_gradient(t->b, t->W, B, t->bx, t->by, t->G, t->sse, t->stream);
             t->t += 1;
             const float b1 = 0.9f, b2 = 0.999f;
             const float c1 = 1.f - std::pow(b1, (float)t->t), c2 = 1.f - std::pow(b2, (float)t->t);
-            adam_kernel<<<256, 256, 0, t->stream>>>(P, t->W, t->G, t->Mom, t->Var, lr, b1, b2, c1, c2, 1e-8f);
+            if (e == cudaSuccess) e = mlp_adam(t->W, t->G, t->Mom, t->Var, lr, b1, b2, c1, c2, 1e-8f, t->stream);
         }
-        last = sse / ((double)t->count * kOut);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(&sse, t->sse, sizeof(double), cudaMemcpyDeviceToHost, t->stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(t->stream);
+        if (e != cudaSuccess) return cuda_fail(nullptr, e, "training step");
     }
-    if (cudaStreamSynchronize(t->stream) != cudaSuccess) return fail(nullptr, RF_ERR_CUDA, "training");
-    if (loss) *loss = (float)last;
+    if (loss) *loss = (float)(sse / ((double)t->count * kOut));
     return RF_OK;
 }
 
@@ -979,12 +788,16 @@ rf_status rf_trainer_loss_grad(rf_trainer *t, const float *features, const float
         return fail(nullptr, RF_ERR_INVALID_ARG, "bad arguments");
     cudaSetDevice(t->device);
     if (!ensure_batch(t, (int)count)) return fail(nullptr, RF_ERR_OOM, "batch buffers");
-    cudaMemcpy(t->bx, features, sizeof(float) * count * kIn, cudaMemcpyHostToDevice);
-    cudaMemcpy(t->by, targets, sizeof(float) * count * kOut, cudaMemcpyHostToDevice);
     double sse = 0.0;
-    cudaError_t e = forward_backward(t, (int)count, &sse);
+    cudaError_t e = cudaMemcpyAsync(t->bx, features, sizeof(float) * count * kIn, cudaMemcpyHostToDevice, t->stream);
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(t->by, targets, sizeof(float) * count * kOut, cudaMemcpyHostToDevice, t->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(t->sse, 0, sizeof(double), t->stream);
+    if (e == cudaSuccess) e = mlp_gradient(t->b, t->W, (int)count, t->bx, t->by, t->G, t->sse, t->stream);
     if (e == cudaSuccess && grad)
-        e = cudaMemcpy(grad, t->G, sizeof(float) * MlpLayout().total, cudaMemcpyDeviceToHost);
+        e = cudaMemcpyAsync(grad, t->G, sizeof(float) * MlpLayout().total, cudaMemcpyDeviceToHost, t->stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&sse, t->sse, sizeof(double), cudaMemcpyDeviceToHost, t->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(t->stream);
     if (e != cudaSuccess) return cuda_fail(nullptr, e, "loss/grad");
     if (loss) *loss = (float)(sse / ((double)count * kOut));
     return RF_OK;
