@@ -45,7 +45,7 @@ void free_all(rf_handle *h) {
         cudaFree(h->V[i]);
         cudaFree(h->W[i]);
     }
-    void *ptrs[] = {h->tab, h->A64, h->LU, h->lu_r, h->lu_piv, h->lu_info, h->mfpart, h->mvx, h->A32, h->A16, h->b, h->x, h->bpart, h->velpart, h->PV64, h->PW64,
+    void *ptrs[] = {h->tab, h->A64, h->LU, h->lu_r, h->lu_piv, h->lu_info, h->mfpart, h->mvx, h->A32, h->A16, h->b, h->x, h->PV64, h->PW64,
                     h->PV32, h->PW32, h->vpart, h->pvx, h->pwx, h->work64, h->work32, h->r64, h->r32,
                     h->d32, h->x32, h->Pblocks, h->knn, h->mlp_w, h->mlp_wtc, h->mlp_err, h->feat, h->mlp_h1, h->mlp_h2, h->mlp_out,
                     h->dscal, h->rb.partials, h->rb.counter, h->near_bits, h->near_list, h->near_cnt,
@@ -439,7 +439,6 @@ rf_status rf_create(const rf_params *p, const double *positions, const double *o
     CKC(dalloc(&h->x, h->n), "alloc x");
     CKC(cudaMemset(h->x, 0, h->n * 8), "memset x");
     CKC(cudaMemset(h->b, 0, h->n * 8), "memset b");
-    CKC(dalloc(&h->bpart, (size_t)h->asm_chunks * h->n_loc), "alloc rhs partials");
     // the split assembly (FP32 far pairs, FP64 near pairs) for the reduced
     // precisions with analytic integration; near_field_c >= 1e30 asks for FP64
     // integrals everywhere and keeps the tile kernel
@@ -461,7 +460,6 @@ rf_status rf_create(const rf_params *p, const double *positions, const double *o
             CKC(dalloc(&h->near_contr, (size_t)M * 3 * (N + 1)), "alloc rhs partials");
         }
     }
-    CKC(dalloc(&h->velpart, (size_t)h->vel_chunks * 6 * M), "alloc velocity partials");
     if (p->velocity_mode == RF_VEL_REUSE) {
         const size_t psz = (size_t)h->ldp * (size_t)h->n;
         if (prec == RF_PREC_FP64) {
@@ -483,8 +481,16 @@ rf_status rf_create(const rf_params *p, const double *positions, const double *o
     h->work_elems = std::max({rf::gemv_work_elems(h->lda, h->sm_count, 8), rf::gemv_work_elems(h->lda, h->sm_count, 4),
                               rf::gemv_work_elems(h->lda, h->sm_count, 2), rf::gemv_work_elems(h->ldp, h->sm_count, 8),
                               rf::gemv_work_elems(h->ldp, h->sm_count, 4)});
-    CKC(dalloc(&h->work64, h->work_elems), "alloc matvec workspace");
-    CKC(dalloc(&h->work32, h->work_elems), "alloc matvec workspace");
+    const int64_t gemv_elems = h->work_elems;
+    // One FP64 workspace for what lives within one call: the products' partial
+    // sums, the assembly's and the velocities' per-chunk sums, the single-kernel
+    // GMRES of small systems (a small handle's creation is mostly its allocations)
+    h->small = prec == RF_PREC_FP64 && shards == 1 && rf::gmres_small_supported(h->n, p->gmres_restart, h->sm_count);
+    h->work_elems = std::max({h->work_elems, (int64_t)h->asm_chunks * h->n_loc, (int64_t)h->vel_chunks * 6 * M,
+                              h->small ? rf::gmres_small_work(h->n, h->sm_count) : 0});
+    CKC(dalloc(&h->work64, h->work_elems), "alloc workspace");
+    h->bpart = h->velpart = h->work64;
+    if (prec != RF_PREC_FP64) CKC(dalloc(&h->work32, gemv_elems), "alloc matvec workspace");
     CKC(dalloc(&h->dscal, 8), "alloc scalars");
     CKC(cudaMallocHost(&h->hscal, 8 * sizeof(double)), "alloc pinned scalars");
     h->rb.max_blocks = 1024;
@@ -817,7 +823,39 @@ rf_status rf_solve_system(rf_handle *h) {
         };
         rf::Gmres<double>::Op A = [&A_s](const double *in, double *out) { return A_s(in, out, nullptr); };
         rf::Gmres<double>::Op P = [&P_s](const double *in, double *out) { return P_s(in, out, nullptr); };
-        {
+        bool done = false;
+        if (h->small && !use_pc && !h->gt.on) {
+            // the whole solve in one kernel (one shard holds the whole system, with a communicator or without)
+            rf::SmallGmresArgs sa{};
+            sa.A = h->A64;
+            sa.lda = h->lda;
+            sa.n = h->n;
+            sa.m = m;
+            sa.max_iters = maxit > 0 ? maxit : (int)h->n;
+            sa.tol = tol;
+            sa.b = h->b;
+            sa.x = h->x;
+            sa.barrier = reinterpret_cast<unsigned *>(h->dscal + 2);
+            sa.stat = reinterpret_cast<rf::SmallGmresStat *>(h->dscal + 3);
+            const cudaError_t e = rf::launch_gmres_small(sa, h->work64, h->sm_count, st);
+            if (e != cudaErrorCooperativeLaunchTooLarge) {
+                CK(h, e, "GMRES");
+                rf::SmallGmresStat *hs = reinterpret_cast<rf::SmallGmresStat *>(h->hscal);
+                CK(h, cudaMemcpyAsync(hs, sa.stat, sizeof(*hs), cudaMemcpyDeviceToHost, st), "GMRES");
+                CK(h, cudaStreamSynchronize(st), "GMRES");
+                if (hs->info == rf::kSmallTimeout)
+                    return rf::fail(h, RF_ERR_DEVICE_TIMEOUT, "GMRES: a grid barrier timed out");
+                res.info = hs->info == rf::kSmallNaN ? rf::kInfoNaN : hs->info == rf::kSmallBudget ? rf::kInfoBudget : 0;
+                res.iterations = hs->iterations;
+                res.matvecs = hs->matvecs;
+                res.backward_error = hs->backward_error;
+                res.launches = 1;
+                done = true;
+            } else {
+                cudaGetLastError();  // fewer SMs to this process than the device has
+            }
+        }
+        if (!done) {
             bool pc_on = use_pc;
             double prev = 1.0;  // residual relative to |b| before this trial
             rf::GmresResult part;

@@ -8,7 +8,7 @@
 // step queued after the stop costs a few empty launches.  The inner solves of
 // the mixed-precision refinement and the FP64 and FP32 GMRES all run this way
 // (restart lengths up to kArnoldiMax; longer ones use the host-controlled
-// solver).  What bounds a small system is the number of dependent launches: a
+// solver; small FP64 systems run in one kernel, gmres_small.cu).  What bounds a small system is the number of dependent launches: a
 // step is the product's two kernels, three orthogonalisation passes and one
 // scaling, where the host-controlled solver takes j + 5 launches, a copy and
 // a wait of the host.  Whole time steps,

@@ -47,11 +47,11 @@ struct rf_handle {
     int64_t a_plane = 0;
     double *b = nullptr;       // right-hand side
     double *x = nullptr;       // coefficients (warm start for the next solve)
-    double *bpart = nullptr;   // [nchunks][n]
+    double *bpart = nullptr;   // [nchunks][n] (work64)
     int asm_chunks = 1, asm_chunk = 1;
     bool asm64 = false;        // FP64 analytic assembly by autonomous warps (assemble64.cu)
     int vel_chunks = 1, vel_chunk = 1;
-    double *velpart = nullptr; // [vel_chunks][6M]
+    double *velpart = nullptr; // [vel_chunks][6M] (work64)
     double *mvx = nullptr;     // [2n] operand and result of rf_matvec (and of rf_matvec_free), made at their first use
     double *mfpart = nullptr;  // [vel_chunks][n] matrix-free product partials where work64 is too small
     // velocity panels (reuse mode)
@@ -71,9 +71,10 @@ struct rf_handle {
     double *far_contr = nullptr, *near_contr = nullptr;
     double *pvx = nullptr, *pwx = nullptr;
     // matvec workspace
-    double *work64 = nullptr;
+    double *work64 = nullptr;  // FP64 partial sums that live within one call
     float *work32 = nullptr;
     int64_t work_elems = 0;
+    bool small = false;        // small FP64 system: GMRES in one kernel (gmres_small.cu), in work64 and dscal[2..5]
     // solver
     std::unique_ptr<rf::Gmres<double>> gm64;
     std::unique_ptr<rf::Gmres<float>> gm32;

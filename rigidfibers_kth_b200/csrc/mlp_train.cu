@@ -317,6 +317,8 @@ cudaError_t layer(const LayerArgs &g, int *ctas, cudaStream_t st) {
 
 }  // namespace
 
+int mlp_slices(int rows) { return std::max(1, std::min(8, rows / 128)); }
+
 int mlp_loss_parts(int rows) { return ((rows + 31) / 32) * ((kMlpOut + 31) / 32); }
 
 cudaError_t mlp_gradient(const MlpBatch &b, const float *W, int rows, const float *X, const float *Y, float *G,
@@ -344,7 +346,7 @@ cudaError_t mlp_gradient(const MlpBatch &b, const float *W, int rows, const floa
     if ((e = layer<false, kMask>(g, &ctas, st)) != cudaSuccess) return e;
     GradArgs w{};
     w.rows = rows;
-    const int slices = std::max(1, std::min(kMlpSlices, rows / 64));
+    const int slices = mlp_slices(rows);
     w.per = ((rows + slices - 1) / slices + kBK - 1) / kBK * kBK;
     w.part = b.part;
     w.params = L.total;

@@ -11,7 +11,6 @@ namespace rf {
 
 constexpr int kMlpIn = RF_MLP_IN, kMlpHid = RF_MLP_HIDDEN, kMlpOut = RF_MLP_OUT;
 constexpr int kMlpOutLd = (kMlpOut + 3) / 4 * 4;  // rows of dO start on 16 bytes
-constexpr int kMlpSlices = 16;                    // most slices of a batch's weight gradients
 
 // parameter offsets inside the packed weight vector
 struct MlpLayout {
@@ -22,10 +21,11 @@ struct MlpLayout {
 // A batch's intermediate results (device; 16-byte aligned)
 struct MlpBatch {
     float *h1, *h2, *dO, *dh2, *dh1;   // rows x 256, rows x 256, rows x kMlpOutLd, rows x 256, rows x 256
-    float *part;                       // [kMlpSlices][params]
+    float *part;                       // [mlp_slices(rows)][params]
     double *sse;                       // mlp_loss_parts(rows)
 };
 int mlp_loss_parts(int rows);
+int mlp_slices(int rows);   // slices of a batch's weight gradients, not falling with the rows
 
 // G = the gradient of mean (o - Y)^2 over the rows' 225 outputs, *sse += sum
 // (o - Y)^2 (device).

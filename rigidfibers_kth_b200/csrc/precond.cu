@@ -643,7 +643,6 @@ rf_status rf_trainer_create(int32_t device, uint64_t seed, rf_trainer **out) {
     bool ok = cudaStreamCreateWithFlags(&t->stream, cudaStreamNonBlocking) == cudaSuccess &&
               cudaMalloc(&t->W, sizeof(float) * P) == cudaSuccess && cudaMalloc(&t->G, sizeof(float) * P) == cudaSuccess &&
               cudaMalloc(&t->Mom, sizeof(float) * P) == cudaSuccess && cudaMalloc(&t->Var, sizeof(float) * P) == cudaSuccess &&
-              cudaMalloc(&t->b.part, sizeof(float) * P * kMlpSlices) == cudaSuccess &&
               cudaMalloc(&t->sse, sizeof(double)) == cudaSuccess;
     if (!ok) {
         rf_trainer_destroy(t);
@@ -670,8 +669,7 @@ rf_status rf_trainer_create(int32_t device, uint64_t seed, rf_trainer **out) {
 rf_status rf_trainer_destroy(rf_trainer *t) {
     if (!t) return RF_ERR_INVALID_ARG;
     cudaSetDevice(t->device);
-    void *ptrs[] = {t->W, t->G, t->Mom, t->Var, t->X, t->Y, t->bx, t->by, t->b.h1, t->b.h2, t->b.dO, t->b.dh2,
-                    t->b.dh1, t->b.part, t->b.sse, t->perm, t->sse};
+    void *ptrs[] = {t->W, t->G, t->Mom, t->Var, t->X, t->Y, t->bx, t->perm, t->sse};
     for (void *p : ptrs) cudaFree(p);
     if (t->stream) cudaStreamDestroy(t->stream);
     delete t;
@@ -707,21 +705,27 @@ rf_status rf_trainer_add_samples(rf_trainer *t, const float *features, const flo
 }
 
 namespace {
+// Buffers of a batch, one allocation (its first float is bx).
 bool ensure_batch(rf_trainer *t, int B) {
     if (B <= t->bcap) return true;
-    void *ptrs[] = {t->bx, t->by, t->b.h1, t->b.h2, t->b.dO, t->b.dh2, t->b.dh1, t->b.sse};
-    for (void *p : ptrs) cudaFree(p);
-    auto f = [](float **p, int64_t n) {
-        *p = nullptr;
-        return cudaMalloc(p, sizeof(float) * n) == cudaSuccess;
-    };
-    t->b.sse = nullptr;
+    cudaFree(t->bx);
     const int64_t n = B;
-    const bool ok = f(&t->bx, n * kIn) & f(&t->by, n * kOut) & f(&t->b.h1, n * kHid) & f(&t->b.h2, n * kHid) &
-                    f(&t->b.dO, n * kMlpOutLd) & f(&t->b.dh2, n * kHid) & f(&t->b.dh1, n * kHid) &
-                    (cudaMalloc(&t->b.sse, sizeof(double) * mlp_loss_parts(B)) == cudaSuccess);
+    const int64_t sizes[] = {n * kIn, n * kOut, n * kHid, n * kHid, n * kMlpOutLd, n * kHid, n * kHid,
+                             mlp_slices(B) * MlpLayout().total, 2 * (int64_t)mlp_loss_parts(B)};
+    float *sse = nullptr;
+    float **to[] = {&t->bx, &t->by, &t->b.h1, &t->b.h2, &t->b.dO, &t->b.dh2, &t->b.dh1, &t->b.part, &sse};
+    int64_t total = 0;
+    for (int64_t s : sizes) total += (s + 3) / 4 * 4;  // each on 16 bytes
+    float *p = nullptr;
+    t->bcap = 0;
+    const bool ok = cudaMalloc(&p, sizeof(float) * total) == cudaSuccess;
     if (!ok) cudaGetLastError();
-    t->bcap = ok ? B : 0;
+    for (int i = 0; i < 9; ++i) {
+        *to[i] = ok ? p : nullptr;
+        if (ok) p += (sizes[i] + 3) / 4 * 4;
+    }
+    t->b.sse = reinterpret_cast<double *>(sse);
+    if (ok) t->bcap = B;
     return ok;
 }
 }  // namespace

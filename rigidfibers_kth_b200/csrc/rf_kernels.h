@@ -329,4 +329,29 @@ cudaError_t launch_arnoldi_orthogonalize(int64_t n, T *w, T *V, int j, int m, Ar
 template <typename T>
 cudaError_t launch_arnoldi_combine(int64_t n, const T *V, ArnoldiCtrl *c, T *u, cudaStream_t st);
 
+// ---- GMRES(m) of a small FP64 system in one cooperative kernel (gmres_small.cu)
+constexpr int kSmallRows = 64;       // rows of a CTA at most
+constexpr int kSmallMaxN = 8192;
+enum SmallGmresInfo { kSmallOk, kSmallBudget, kSmallNaN, kSmallTimeout };
+struct SmallGmresStat {
+    int info, iterations, matvecs, pad;
+    double backward_error;
+};
+struct SmallGmresArgs {
+    const double *A;          // n x n, column-major; lda = n rounded up to 64, padding rows zero
+    int64_t lda, n;
+    int m, max_iters;         // restart length (<= kArnoldiMax), step budget
+    double tol;
+    const double *b;
+    double *x;                // the initial guess, then the solution
+    unsigned *barrier;        // device word
+    SmallGmresStat *stat;     // device
+    // set by the launcher
+    int tiles, splits, cols;
+    double *part, *dots, *w, *xcur;
+};
+bool gmres_small_supported(int64_t n, int m, int sm_count);
+int64_t gmres_small_work(int64_t n, int sm_count);   // doubles of `work`
+cudaError_t launch_gmres_small(SmallGmresArgs a, double *work, int sm_count, cudaStream_t st);
+
 }  // namespace rf

@@ -59,3 +59,45 @@ def test_warm_start_zero_rhs_and_true_residual(precision, tol):
         assert np.abs(b).max() == 0.0
         assert sim.solve_system() == 0
         assert np.abs(sim.coeffs()).max() == 0.0
+
+
+# one CTA's rows and the next (148 rows a fiber pair more or less), ragged
+# 64-row tiles, the largest system of the single-kernel solver and the first
+# beyond it (N = 4: 12 rows a fiber, 8184 and 8196); the product timer takes the
+# kernel-per-pass solver on the same system
+@pytest.mark.parametrize("M,N,restart", [(9, 5, 10), (10, 5, 10), (43, 1, 7), (50, 3, 16), (682, 4, 10), (683, 4, 10)])
+def test_single_kernel_solver_matches_launched_passes(M, N, restart):
+    pos, ori = rf.generate_layout(M, "gaussian", 3.0 * (M / 1000.0) ** (1 / 3), 0.2, seed=M)
+    p = rf.FiberParams(slenderness=1e-3, num_terms_in_force_expansion=N, gmres_restart=restart, gmres_tol=1e-11,
+                       gmres_max_iters=300)
+    with rf.Simulation(rf.Configuration(p, pos, ori)) as sim:
+        sim.assemble_system()
+        out = []
+        for timed in (False, True):
+            sim.set_history(pos, ori, pos, ori, np.zeros(3 * N * M))
+            sim.gemv_timer(timed)
+            assert sim.solve_system() == 0
+            out.append((sim.coeffs(), sim.solve_stats()))
+    (x, a), (y, b) = out
+    assert a["iterations"] == b["iterations"] and a["matvecs"] == b["matvecs"]
+    # the same steps; sums of n products and n squares in another order: a few n
+    # units of rounding of |x|, far below 1e-11
+    assert np.abs(x - y).max() <= 1e-11 * np.abs(y).max()
+
+
+def test_one_rank_communicator_above_the_single_kernel_solver():
+    """A system too large for the single-kernel solver: every product of a
+    one-rank sharded handle goes through the all-gather and the compaction, and
+    steps exactly like the whole system's."""
+    M = 560
+    pos, ori = rf.generate_layout(M, "gaussian", 2.0, 0.2, seed=2103)
+    out = []
+    for sharded in (False, True):
+        kw = dict(nccl_id=rf.shard_unique_id()) if sharded else {}
+        p = rf.FiberParams(slenderness=1e-3, gmres_tol=1e-10, gmres_max_iters=300, shard_index=0, shard_count=1)
+        with rf.Simulation(rf.Configuration(p, pos, ori), **kw) as s:
+            for t in range(2):
+                assert s.step(t) == 0
+            out.append(s.state() + s.velocities() + (s.coeffs(), s.rhs()))
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
