@@ -41,33 +41,14 @@
 // loads).
 #include <algorithm>
 
+#include "pair_block64.cuh"
 #include "rf_kernels.h"
 
 namespace rf {
 
 namespace {
 
-constexpr int kTI = 4;      // targets per warp
 constexpr int kWarps = 4;   // warps per CTA
-
-template <int N>
-struct Dims64 {
-    static constexpr int NL = N + 1;
-    static constexpr int NU = N + 1, NV = N + 3;
-    static constexpr int NC = NU + NV;              // scalars per point
-    static constexpr int COLS = kTI * NC;           // product columns: a multiple of 8
-    static constexpr int TILES = COLS / 8;
-    static constexpr int KST = 9;                   // stride of a scalar's projections (8 rows)
-    static constexpr int PST = NC * KST + (NC * KST % 16 <= 6 ? 6 : 22) - NC * KST % 16;  // of a pair's: 6 mod 16
-    static constexpr int TH = kTI * PST;
-    static constexpr int RT = kTI * 3 * N;          // staged rows
-    static constexpr int CT = 3 * N;                // staged columns
-    static constexpr int PAN = 2 * CT * kTI * 3;    // staged panel entries
-};
-
-// points of a row of G: a stride of 4 mod 8 keeps the tensor-core operand
-// loads and the point-order stores free of bank conflicts
-__host__ __device__ constexpr int ldq_of(int LQ) { return ((LQ + 3) / 8) * 8 + 4; }
 
 // shared memory of a warp, in doubles: G, or the projections, the staged block
 // and the staged panels; then the targets, the right-hand-side sums and the
@@ -83,22 +64,6 @@ template <int N, bool PANELS>
 __host__ __device__ constexpr int warp_doubles(int LQ) {
     return region_doubles<N, PANELS>(LQ) + kTI * 6 + kTI * (N + (PANELS ? 2 : 0)) * 3 + kTI * kMaxLQ / 8;
 }
-
-// Coefficients of row k of the factored block: <s f>_k and <s^2 f>_k from
-// rows k - 2 .. k + 2 (Bonnet), and v = g1 (AI I + D X^T + p Z^T) +
-// t (g1 Y + g2 Q)^T.
-struct RowTab {
-    double al, be;        // <s f>_k = al f_{k+1} + be f_{k-1}
-    double c2p, c20, c2m; // <s^2 f>_k = c2p f_{k+2} + c20 f_k + c2m f_{k-2}
-    double g1, g2;
-};
-
-struct GStoreUV {
-    double *g;   // column 0 of the point's pair, at the point
-    int ldq, nu;
-    __device__ __forceinline__ void u(int p, double v) const { g[p * ldq] = v; }
-    __device__ __forceinline__ void v(int p, double v) const { g[(nu + p) * ldq] = v; }
-};
 
 // LQC: the points per fiber when known at compile time (24, the usual 8 x 3), else 0
 template <int N, bool PANELS, int KSMAX, int LQC>
@@ -131,30 +96,8 @@ __global__ void __launch_bounds__(kWarps * 32, 4) assemble64_kernel(AsmArgs a) {
         const int m = t / kMaxLQ, q = t % kMaxLQ;
         s_wP[t] = (m <= N + 2 && q < LQ) ? tab.wv[q] * tab.P[m][q] : 0.0;
     }
-    if (tid < NL + 2) {
-        const int k = tid < NL ? tid : tid - NL;
-        auto al = [](int r) { return (r + 1.0) / (2.0 * r + 1.0); };
-        auto be = [](int r) { return r / (2.0 * r + 1.0); };
-        RowTab r;
-        r.al = al(k);
-        r.be = be(k);
-        r.c2p = al(k) * al(k + 1);
-        r.c20 = al(k) * be(k + 1) + (k > 0 ? be(k) * al(k - 1) : 0.0);
-        r.c2m = k > 1 ? be(k) * be(k - 1) : 0.0;
-        if (tid < NL) {
-            r.g1 = k >= 2 ? tab.gamma[k] : 0.0;
-            r.g2 = k >= 2 ? -tab.gamma[k] * tab.Ek[k] : tab.D1;
-        } else {
-            r.g1 = (k == 0 ? 0.5 : 1.5) / tab.d;
-            r.g2 = k == 0 ? 0.0 : -1.5 / tab.d;
-        }
-        s_row[tid] = r;
-    }
+    block_tables<N>(tab, s_row, s_leg, tid);
     for (int t = tid; t < Far<N>::kCoef; t += kWarps * 32) s_far[t] = Far<N>::coef(t);
-    if (tid < NL * 3) {
-        const int m = tid / 3, p = m - 2 * (tid % 3);
-        s_leg[tid] = p >= 0 ? leg_scale(m) * leg_coef(m, p) : 0.0;
-    }
     __syncthreads();
     // tensor-core A operands: lane holds w_q P_row(q), row = lane / 4, q = 4 s + lane % 4
     double afrag[KSMAX];
@@ -235,82 +178,19 @@ __global__ void __launch_bounds__(kWarps * 32, 4) assemble64_kernel(AsmArgs a) {
         }
         __syncwarp();
         // ---------------- P2
-        {
-            double d[D::TILES][2];
-#pragma unroll
-            for (int t = 0; t < D::TILES; ++t) d[t][0] = d[t][1] = 0.0;
-            const double *bsrc = s_g + (lane >> 2) * LDQ + (lane & 3);
-#pragma unroll
-            for (int s = 0; s < KSMAX; ++s)
-                if (s < KS) {
-#pragma unroll
-                    for (int t = 0; t < D::TILES; ++t)
-                        dmma_8x8x4(d[t][0], d[t][1], afrag[s], bsrc[t * 8 * LDQ + 4 * s], d[t][0], d[t][1]);
-                }
-            __syncwarp();  // every lane's operands read: the projections take the place of G
-#pragma unroll
-            for (int t = 0; t < D::TILES; ++t) {
-                const int cc = t * 8 + 2 * (lane & 3);  // even: both columns are of one pair
-                double *o = s_th + cc / NC * D::PST + cc % NC * KST + (lane >> 2);
-                o[0] = d[t][0];
-                o[KST] = d[t][1];
-            }
-        }
-        __syncwarp();
-        // ---------------- P3: rows k in turn, the projections of rows k - 2 .. k + 2 kept in registers
+        project_pairs<N, KSMAX>(s_g, s_th, afrag, LDQ, KS, lane);
+        // ---------------- P3
         if (item3) {
-            const double *x = s_tgt + ti3 * 6;
-            const double t0 = x[3], t1 = x[4], t2 = x[5];
-            const double D0 = x[0] - xs[0], D1 = x[1] - xs[1], D2 = x[2] - xs[2];
-            const double dt = D0 * t0 + D1 * t1 + D2 * t2, tt = t0 * t0 + t1 * t1 + t2 * t2,
-                         pt = ts[0] * t0 + ts[1] * t1 + ts[2] * t2;
-            const double l0 = s_leg[3 * m3], l1 = s_leg[3 * m3 + 1], l2 = s_leg[3 * m3 + 2];
-            const double *U = s_th + ti3 * D::PST + m3 * KST, *V = U + NU * KST;
-            const int o1 = (max(m3 - 2, 0) - m3) * KST, o2 = (max(m3 - 4, 0) - m3) * KST;
-            // Legendre combination m of the scalars at f, f - 2, f - 4
-            auto leg = [&](const double *f) { return fma(l2, f[o2], fma(l1, f[o1], l0 * f[0])); };
-            double r0m2, r0m1 = 0.0, r0 = 0.0, r0p1 = leg(V), r0p2 = leg(V + 1);         // <cRR>, rows k-2 .. k+2
-            double c0m1, c0 = 0.0, c0p1 = leg(V + KST);                                  // -<cPR>, rows k-1 .. k+1
             const bool own = ti3 == self;
             double *dst = s_blk + 3 * (m3 - 1) * D::RT + ti3 * 3 * N;
             double *dpan = s_pan + 3 * (m3 - 1) * (kTI * 3) + ti3 * 3;
             double *acc = s_acc + ti3 * ACCN * 3;
-#pragma unroll 1
-            for (int k = 0; k <= N; ++k) {
-                r0m2 = r0m1; r0m1 = r0; r0 = r0p1; r0p1 = r0p2; r0p2 = leg(V + k + 2);
-                c0m1 = c0; c0 = c0p1; c0p1 = leg(V + KST + k + 1);
-                if (!PANELS && k == 0) continue;
-                const double E = leg(V + 2 * KST + k), AI = leg(U + k);
-                const RowTab *rt = s_row + k;
-                const double al = rt->al, be = rt->be;
-                const double R1 = fma(al, r0p1, be * r0m1);
-                const double R2 = fma(rt->c2p, r0p2, fma(rt->c20, r0, rt->c2m * r0m2));
-                const double C0 = -c0, C1 = -fma(al, c0p1, be * c0m1);
-                const double X0 = fma(r0, D0, fma(R1, t0, C0 * ts[0])), X1 = fma(r0, D1, fma(R1, t1, C0 * ts[1])),
-                             X2 = fma(r0, D2, fma(R1, t2, C0 * ts[2]));
-                const double Y0 = fma(R1, D0, fma(R2, t0, C1 * ts[0])), Y1 = fma(R1, D1, fma(R2, t1, C1 * ts[1])),
-                             Y2 = fma(R1, D2, fma(R2, t2, C1 * ts[2]));
-                const double Z0 = fma(C0, D0, fma(C1, t0, E * ts[0])), Z1 = fma(C0, D1, fma(C1, t1, E * ts[1])),
-                             Z2 = fma(C0, D2, fma(C1, t2, E * ts[2]));
-                // Q = theta t
-                const double Q0 = fma(AI, t0, fma(dt, X0, fma(tt, Y0, pt * Z0))),
-                             Q1 = fma(AI, t1, fma(dt, X1, fma(tt, Y1, pt * Z1))),
-                             Q2 = fma(AI, t2, fma(dt, X2, fma(tt, Y2, pt * Z2)));
-                // g1 theta + g2 t Q^T to out (l >= 1), or its product with f added to sum (l = 0)
+            block_rows<N, PANELS>(s_row, s_leg, s_th + ti3 * D::PST + m3 * KST, m3, s_tgt + ti3 * 6, xs, ts,
+                                  [&](int k, const BlockRow &r) {
+                // the block to out (l >= 1), or its product with f added to sum (l = 0)
                 auto block = [&](double g1, double g2, double *out, int ldo, double *sum, bool identity) {
-                    const double y0 = fma(g1, Y0, g2 * Q0), y1 = fma(g1, Y1, g2 * Q1), y2 = fma(g1, Y2, g2 * Q2);
-                    const double gD0 = g1 * D0, gD1 = g1 * D1, gD2 = g1 * D2;
-                    const double gp0 = g1 * ts[0], gp1 = g1 * ts[1], gp2 = g1 * ts[2], gA = g1 * AI;
-                    double v[9];  // [column][row]
-                    v[0] = fma(gD0, X0, fma(t0, y0, fma(gp0, Z0, gA)));
-                    v[1] = fma(gD1, X0, fma(t1, y0, gp1 * Z0));
-                    v[2] = fma(gD2, X0, fma(t2, y0, gp2 * Z0));
-                    v[3] = fma(gD0, X1, fma(t0, y1, gp0 * Z1));
-                    v[4] = fma(gD1, X1, fma(t1, y1, fma(gp1, Z1, gA)));
-                    v[5] = fma(gD2, X1, fma(t2, y1, gp2 * Z1));
-                    v[6] = fma(gD0, X2, fma(t0, y2, gp0 * Z2));
-                    v[7] = fma(gD1, X2, fma(t1, y2, gp1 * Z2));
-                    v[8] = fma(gD2, X2, fma(t2, y2, fma(gp2, Z2, gA)));
+                    double v[9];
+                    r.entries(g1, g2, v);
                     if (own) {  // the fiber itself: the identity in A, nothing else
 #pragma unroll
                         for (int e = 0; e < 9; ++e) v[e] = e % 4 == 0 && identity ? 1.0 : 0.0;
@@ -324,12 +204,11 @@ __global__ void __launch_bounds__(kWarps * 32, 4) assemble64_kernel(AsmArgs a) {
                         for (int e = 0; e < 3; ++e) sum[e] += fma(v[e], f0, fma(v[3 + e], f1, v[6 + e] * f2));
                     }
                 };
-                if (k > 0) block(rt->g1, rt->g2, dst + 3 * (k - 1), D::RT, acc + 3 * (k - 1), k == m3);
-                if (PANELS && k < 2) {
-                    const RowTab *rp = s_row + NL + k;
-                    block(rp->g1, rp->g2, dpan + k * D::CT * kTI * 3, kTI * 3, acc + 3 * (N + k), false);
-                }
-            }
+                if (k > 0) block(s_row[k].g1, s_row[k].g2, dst + 3 * (k - 1), D::RT, acc + 3 * (k - 1), k == m3);
+                if (PANELS && k < 2)
+                    block(s_row[NL + k].g1, s_row[NL + k].g2, dpan + k * D::CT * kTI * 3, kTI * 3, acc + 3 * (N + k),
+                          false);
+            });
         }
         __syncwarp();
         // ---------------- P4: two consecutive rows per lane

@@ -23,8 +23,9 @@
 //                     its two 16-bit planes where stored so) and the
 //                     velocity-panel rows in shared memory, and one lane
 //                     hands whole column segments to the copy engine;
-//   near_pairs_kernel FP64, one warp per near pair: lane = Gauss point, the
-//                     projection on the FP64 tensor cores (mma.sync m8n8k4).
+//   near_pairs_kernel FP64, a warp per four near pairs of a target, their
+//                     points integrated together, the projection on the FP64
+//                     tensor cores (mma.sync m8n8k4), as in assemble64.cu.
 // A finish kernel sums the per-chunk right-hand-side partials in a fixed order.
 //
 // Projection without forming the tensors.  The reference forms, per target
@@ -43,6 +44,7 @@
 // another order.
 #include <algorithm>
 
+#include "pair_block64.cuh"
 #include "rf_kernels.h"
 
 namespace rf {
@@ -831,210 +833,191 @@ __global__ void __launch_bounds__(32 * RF_FAR_WARPS, RF_FAR_MINB / RF_FAR_WARPS)
 
 // ---------------------------------------------------------------- near pairs (FP64)
 constexpr int kNearWarps = 4;
-#ifndef RF_NEAR_MINB
-#define RF_NEAR_MINB 4
-#endif
-constexpr int kXq = 52;  // q stride of X[col][q]: 52 = 4 mod 16 makes the B fragments conflict-free
-constexpr int kTmLd = 17;  // row stride of the projections Tm[k][col] (odd: rows fall in different banks)
+// A pair's staged record: weight stride 66 floats (even: the copy reads float2),
+// so the 20 lanes (pair, m >= 1) that store an entry use 16 different banks
+constexpr int kNearStage = kNearWeight + 2;
 
 template <int N>
 struct NearSmem {
-    static constexpr int X = 16 * kXq;                  // per-point scalars [col][q], cols >= 2N+4 zero
-    static constexpr int TM = 8 * kTmLd + (8 * kTmLd) % 2;  // projections [k][col] (even: keeps BLK 16-byte aligned)
-    static constexpr int BLK = kNearBlock / 2;          // staged block + panels (floats)
-    static constexpr int RHS = 3 * (N + 1) + 1;
-    static constexpr int WARP = X + TM + BLK + RHS + ((X + TM + BLK + RHS) & 1);
-    static constexpr int TABLES = 8 * kMaxLQ + kMaxLQ + 72 + 32;   // w P, s, Legendre coefficients, row constants
-    // every per-warp region and the staged block (read as float4) start on 16 bytes
-    static_assert(X % 2 == 0 && (X + TM) % 2 == 0 && WARP % 2 == 0 && TABLES % 2 == 0, "16-byte alignment");
-    static size_t bytes() { return sizeof(double) * (TABLES + (size_t)kNearWarps * WARP); }
+    using D = Dims64<N>;
+    static constexpr int NRHS = 3 * (N + 1);
+    static constexpr int PAIR = N * kNearStage;                          // floats of a staged pair
+    static constexpr int THS = (D::TH + 1) / 2 * 2 + kTI * PAIR / 2;     // projections, then the staged records
+    static_assert(kTI * PAIR % 2 == 0, "staged records in doubles");
+    // the scalars G, or what follows them
+    __host__ __device__ static constexpr int region(int LQ) {
+        return ((D::COLS * ldq_of(LQ) > THS ? D::COLS * ldq_of(LQ) : THS) + 1) / 2 * 2;
+    }
+    // region, 4 sources, the warp's right-hand-side sums, the point list
+    __host__ __device__ static constexpr int warp(int LQ) {
+        return region(LQ) + kTI * 6 + kTI * NRHS + kTI * kMaxLQ / 8;
+    }
+    static constexpr int TABLES = kMaxLQ + (N + 3) * (int)(sizeof(RowTab) / sizeof(double)) + 3 * (N + 1) + Far<N>::kCoef + 6;
+    static size_t bytes(int LQ) { return sizeof(double) * (TABLES + 1 + (size_t)kNearWarps * warp(LQ)); }
 };
 
-// One CTA per target fiber, warps over its near sources.  Per pair: lane =
-// Gauss point for the FP64 moments, the projection on the tensor cores, then
-// lane = (source weight m, target row k) for the block entries.  The block
-// goes to the near-pair buffer (DIRECT = false; the far kernel merges it into
-// its column stores) or straight into A (DIRECT = true, used when the buffer
-// could not be grown).
-template <int N, bool PANELS, bool DIRECT>
-__global__ void __launch_bounds__(kNearWarps * 32, RF_NEAR_MINB) near_pairs_kernel(SplitArgs a) {
-    using SD = SplitDims<N>;
+// One CTA per target fiber; a warp takes four of its near sources at a time.
+// The pairs' points are split into those of the backward recursion run to n = 0
+// (far_point) and the rest, which keep the reference's closed forms, so that
+// every warp pass runs one of the two; then projections on the FP64 tensor
+// cores and the block rows as in assemble64.cu, lane = (pair, m).  The four
+// records leave together, consecutive slots, to the near-pair buffer (direct =
+// false; the far kernel merges them into its column stores) or straight into A
+// (direct = true, used when the buffer could not be grown).
+// Bound by FP64 and integer issue (53 % of the issue slots, FP64 pipe 46 %).  One
+// warp per pair (24 of 32 lanes with a point, each running the 26-step backward
+// recursion or the forward one, a 36-way division of the block over 32 lanes)
+// took 2.19 ms for the 460 thousand near pairs of a cloud of 2000 fibers; four
+// pairs per warp take 0.97 ms.
+template <int N, bool PANELS, int KSMAX>
+__global__ void __launch_bounds__(kNearWarps * 32, 4) near_pairs_kernel(SplitArgs a, int direct) {
+    using D = Dims64<N>;
     using SM = NearSmem<N>;
-    constexpr int NL = SD::NL, NV = SD::NV, RB = SD::RB, NRHS = SD::NRHS;
-    constexpr int KSMAX = kMaxLQ / 4;
+    constexpr int NL = D::NL, NC = D::NC, NU = D::NU, KST = D::KST, RB = 3 * N, NRHS = SM::NRHS;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    double *s_wP = reinterpret_cast<double *>(smem_raw);   // [8][kMaxLQ]
-    double *s_pv = s_wP + 8 * kMaxLQ;
-    double *s_leg = s_pv + kMaxLQ;                          // [8][9]: sc_m a_mp (odd row stride)
-    double *s_bon = s_leg + 72;                             // alpha_k, beta_k, gamma_k, E_k (8 each)
-    double *base = s_wP + SM::TABLES + (size_t)warp * SM::WARP;
-    double *X = base;
-    double *Tm = X + SM::X;
-    float *blk = reinterpret_cast<float *>(Tm + SM::TM);    // [col][row] RB*RB, then panels [w][col][a]
-    double *rhs = Tm + SM::TM + SM::BLK;
-
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int LQ = a.LQ, LDQ = ldq_of(LQ), KS = (LQ + 3) / 4;
     const Tables &tab = *a.tab;
-    const int LQ = a.LQ;
-    const int KS = (LQ + 3) / 4;
-    for (int t = threadIdx.x; t < 8 * kMaxLQ; t += blockDim.x) {
-        const int k = t / kMaxLQ, q = t - k * kMaxLQ;
-        s_wP[t] = (k < SD::KW && q < LQ) ? tab.wv[q] * tab.P[k][q] : 0.0;
-    }
-    for (int t = threadIdx.x; t < kMaxLQ; t += blockDim.x) s_pv[t] = t < LQ ? tab.pv[t] : 0.0;
-    for (int t = threadIdx.x; t < 72; t += blockDim.x) {
-        const int m = t / 9, p = t % 9;
-        s_leg[t] = p < 8 ? leg_scale(m) * leg_coef(m, p) : 0.0;
-    }
-    for (int t = threadIdx.x; t < 8; t += blockDim.x) {
-        s_bon[t] = bonnet_a(t);
-        s_bon[8 + t] = bonnet_b(t);
-        s_bon[16 + t] = t <= N ? tab.gamma[t] : 0.0;
-        s_bon[24 + t] = t <= N ? tab.Ek[t] : 0.0;
-    }
-    for (int t = lane; t < SM::X; t += 32) X[t] = 0.0;
-    for (int t = lane; t < NRHS; t += 32) rhs[t] = 0.0;
-    for (int t = lane; t < kNearBlock; t += 32) blk[t] = 0.f;
-    __syncthreads();
+    const int i = blockIdx.x;
 
+    double *s_pv = reinterpret_cast<double *>(smem_raw);            // kMaxLQ
+    RowTab *s_row = reinterpret_cast<RowTab *>(s_pv + kMaxLQ);       // NL block rows, then 2 panel rows
+    double *s_leg = reinterpret_cast<double *>(s_row + NL + 2);      // NL x 3
+    double *s_far = s_leg + NL * 3;                                  // Far<N>::kCoef
+    double *s_x = s_far + Far<N>::kCoef;                             // target centre and direction
+    double *s_warp = s_pv + (SM::TABLES + 1) / 2 * 2;                // 16-byte aligned
+    double *s_wP = s_warp;                                           // 8 x kMaxLQ, until the operands are loaded
+    double *s_g = s_warp + warp * SM::warp(LQ);
+    double *s_th = s_g;                                              // after the projection
+    float *s_rec = reinterpret_cast<float *>(s_th + (D::TH + 1) / 2 * 2);
+    double *s_src = s_g + SM::region(LQ);                            // 4 x (x, t)
+    double *s_acc = s_src + kTI * 6;                                 // 4 x NRHS
+    unsigned char *s_list = reinterpret_cast<unsigned char *>(s_acc + kTI * NRHS);
+
+    for (int t = tid; t < kMaxLQ; t += kNearWarps * 32) s_pv[t] = t < LQ ? tab.pv[t] : 0.0;
+    for (int t = tid; t < 8 * kMaxLQ; t += kNearWarps * 32) {
+        const int m = t / kMaxLQ, q = t % kMaxLQ;
+        s_wP[t] = (m <= N + 2 && q < LQ) ? tab.wv[q] * tab.P[m][q] : 0.0;
+    }
+    block_tables<N>(tab, s_row, s_leg, tid);
+    for (int t = tid; t < Far<N>::kCoef; t += kNearWarps * 32) s_far[t] = Far<N>::coef(t);
+    if (tid < 6) s_x[tid] = tid < 3 ? a.pos[3 * i + tid] : a.ori[3 * i + tid - 3];
+    __syncthreads();
     double afrag[KSMAX];
 #pragma unroll
-    for (int s = 0; s < KSMAX; ++s) afrag[s] = s_wP[(lane >> 2) * kMaxLQ + 4 * s + (lane & 3)];
+    for (int s = 0; s < KSMAX; ++s) afrag[s] = s < KS ? s_wP[(lane >> 2) * kMaxLQ + 4 * s + (lane & 3)] : 0.0;
+    __syncthreads();
 
-    const int i = blockIdx.x;
-    const double xi[3] = {a.pos[3 * i], a.pos[3 * i + 1], a.pos[3 * i + 2]};
-    const double t[3] = {a.ori[3 * i], a.ori[3 * i + 1], a.ori[3 * i + 2]};
-    const double e2 = 2.0 * tab.eps2, e6 = 6.0 * tab.eps2;
-    const double D1 = tab.D1, sv = 0.5 / tab.d, sw = 1.5 / tab.d;
-    const double *f = tab.half_force;
+    const double eps2 = tab.eps2;
     const int cnt = a.near_cnt[i];
     const int *list = a.near_list + (int64_t)i * a.M;
-    const int slot0 = a.near_off[i];
+    const int64_t slot0 = a.near_off[i];
+    const int ti3 = lane / NL, m3 = lane - ti3 * NL;
+    for (int e = lane; e < kTI * NRHS; e += 32) s_acc[e] = 0.0;
 
-    for (int sidx = warp; sidx < cnt; sidx += kNearWarps) {
-        const int j = list[sidx];
-        const double D[3] = {xi[0] - a.pos[3 * j], xi[1] - a.pos[3 * j + 1], xi[2] - a.pos[3 * j + 2]};
-        const double p[3] = {a.ori[3 * j], a.ori[3 * j + 1], a.ori[3 * j + 2]};
-        // per-point scalars u_p (cols 0..N), v_p (cols N+1..2N+3)
-        for (int q = lane; q < LQ; q += 32) {
-            const double sq = s_pv[q];
-            const double r0x = D[0] + sq * t[0], r0y = D[1] + sq * t[1], r0z = D[2] + sq * t[2];
-            const double b = -2.0 * (p[0] * r0x + p[1] * r0y + p[2] * r0z);
-            const double c = r0x * r0x + r0y * r0y + r0z * r0z;
-            double I[SD::KW], J[SD::KW], S[SD::KW];
+    auto point = [&](int item, double &b, double &c) {
+        const int ti = item / LQ, q = item - ti * LQ;
+        const double sq = s_pv[q];
+        const double *y = s_src + ti * 6;
+        const double r0x = (s_x[0] - y[0]) + sq * s_x[3], r0y = (s_x[1] - y[1]) + sq * s_x[4],
+                     r0z = (s_x[2] - y[2]) + sq * s_x[5];
+        b = -2.0 * (y[3] * r0x + y[4] * r0y + y[5] * r0z);
+        c = r0x * r0x + r0y * r0y + r0z * r0z;
+    };
+
+    for (int s0 = warp * kTI; s0 < cnt; s0 += kNearWarps * kTI) {
+        const int npair = min(kTI, cnt - s0);
+        const int npts = npair * LQ;
+        if (lane < kTI * 6) {
+            const int ti = lane / 6, c = lane % 6;
+            // an unused pair repeats the last one's source; its scalars are zero
+            const int j = list[s0 + min(ti, npair - 1)];
+            s_src[lane] = c < 3 ? a.pos[3 * j + c] : a.ori[3 * j + c - 3];
+        }
+        __syncwarp();
+        // the points: far ones listed from the front, the others from the back
+        int nfar = 0, nnear = 0;
+#pragma unroll 1
+        for (int base = 0; base < npts; base += 32) {
+            const int item = base + lane;
+            double b = 0.0, c = 1.0;
+            if (item < npts) point(item, b, c);
+            const bool far = item < npts && far_point(b, c), near = item < npts && !far;
+            const unsigned mf = __ballot_sync(0xffffffffu, far), mn = __ballot_sync(0xffffffffu, near);
+            const unsigned below = (1u << lane) - 1u;
+            if (far) s_list[nfar + __popc(mf & below)] = (unsigned char)item;
+            if (near) s_list[npts - 1 - nnear - __popc(mn & below)] = (unsigned char)item;
+            nfar += __popc(mf);
+            nnear += __popc(mn);
+        }
+        // unused pairs, and the points between LQ and the next multiple of 4, are zero
+        if (npair < kTI)
+            for (int t = lane; t < (kTI - npair) * NC * LDQ; t += 32) s_g[npair * NC * LDQ + t] = 0.0;
+        const int pad = 4 * KS - LQ;
+        for (int t = lane; t < D::COLS * pad; t += 32) s_g[(t / pad) * LDQ + LQ + t % pad] = 0.0;
+        __syncwarp();
+#pragma unroll 1
+        for (int u = lane; u < nfar; u += 32) {
+            const int item = s_list[u], ti = item / LQ;
+            double b, c;
+            point(item, b, c);
+            moments_far_fp64<N>(b, c, eps2, s_far, GStoreUV{s_g + ti * NC * LDQ + item - ti * LQ, LDQ, NU});
+        }
+#pragma unroll 1
+        for (int u = lane; u < nnear; u += 32) {
+            const int item = s_list[npts - 1 - u], ti = item / LQ;
+            double b, c, I[N + 3], J[N + 3], S[N + 3];
+            point(item, b, c);
             moments_near<N>(b, c, I, J, S);
+            double *g = s_g + ti * NC * LDQ + item - ti * LQ;
 #pragma unroll
-            for (int pp = 0; pp < NL; ++pp) X[pp * kXq + q] = I[pp] + e2 * J[pp];
+            for (int p = 0; p <= N; ++p) g[p * LDQ] = I[p] + 2.0 * eps2 * J[p];
 #pragma unroll
-            for (int pp = 0; pp < NV; ++pp) X[(NL + pp) * kXq + q] = J[pp] - e6 * S[pp];
+            for (int p = 0; p <= N + 2; ++p) g[(NU + p) * LDQ] = J[p] - 6.0 * eps2 * S[p];
         }
         __syncwarp();
-        // projections Tm[k][col] = sum_q w_q P_k(s_q) X[col][q] on the FP64 tensor cores
-#pragma unroll
-        for (int tile = 0; tile < 2; ++tile) {
-            double d0 = 0.0, d1 = 0.0;
-#pragma unroll
-            for (int s = 0; s < KSMAX; ++s)
-                if (s < KS) {
-                    const double bf = X[(8 * tile + (lane >> 2)) * kXq + 4 * s + (lane & 3)];
-                    dmma_8x8x4(d0, d1, afrag[s], bf, d0, d1);
+        project_pairs<N, KSMAX>(s_g, s_th, afrag, LDQ, KS, lane);
+        if (ti3 < npair) {
+            const double *y = s_src + ti3 * 6;
+            float *rec = s_rec + ti3 * SM::PAIR + (m3 - 1) * kNearStage;
+            double *acc = s_acc + ti3 * NRHS;
+            const double f0 = tab.half_force[0], f1 = tab.half_force[1], f2 = tab.half_force[2];
+            block_rows<N, true>(s_row, s_leg, s_th + ti3 * D::PST + m3 * KST, m3, s_x, y, y + 3,
+                                [&](int k, const BlockRow &r) {
+                if (m3 == 0) {  // theta^k_0 f
+                    const double Xf = r.X0 * f0 + r.X1 * f1 + r.X2 * f2, Yf = r.Y0 * f0 + r.Y1 * f1 + r.Y2 * f2,
+                                 Zf = r.Z0 * f0 + r.Z1 * f1 + r.Z2 * f2;
+                    acc[3 * k] += r.AI * f0 + r.D0 * Xf + r.t0 * Yf + r.p0 * Zf;
+                    acc[3 * k + 1] += r.AI * f1 + r.D1 * Xf + r.t1 * Yf + r.p1 * Zf;
+                    acc[3 * k + 2] += r.AI * f2 + r.D2 * Xf + r.t2 * Yf + r.p2 * Zf;
+                    return;
                 }
-            Tm[(lane >> 2) * kTmLd + 8 * tile + 2 * (lane & 3)] = d0;
-            Tm[(lane >> 2) * kTmLd + 8 * tile + 2 * (lane & 3) + 1] = d1;
+                auto block = [&](const RowTab &rt, float *out, int ld) {
+                    double v[9];
+                    r.entries(rt.g1, rt.g2, v);
+#pragma unroll
+                    for (int e = 0; e < 9; ++e) out[(e / 3) * ld + e % 3] = (float)v[e];
+                };
+                if (k > 0) block(s_row[k], rec + 3 * (k - 1), RB);
+                if (PANELS && k < 2) block(s_row[NL + k], rec + 3 * RB + 9 * k, 3);
+            });
         }
         __syncwarp();
-        const double Dt = D[0] * t[0] + D[1] * t[1] + D[2] * t[2];
-        const double tt = t[0] * t[0] + t[1] * t[1] + t[2] * t[2];
-        const double pt = p[0] * t[0] + p[1] * t[1] + p[2] * t[2];
-        // one (weight m, row k) per thread: the N*(N+1) pairs with m >= 1 first,
-        // then the N+1 right-hand-side rows of weight 0 (cheaper) in what is left
-        for (int u = lane; u < NL * NL; u += 32) {
-            const int m = u < N * NL ? u / NL + 1 : 0;
-            const int k = u < N * NL ? u - (m - 1) * NL : u - N * NL;
-            const double *lg = s_leg + m * 9;
-            // coefficient sets of weight m at rows k-2..k+2
-            double AI = 0.0, E = 0.0, R0[5] = {0, 0, 0, 0, 0}, C0[3] = {0, 0, 0};
-            for (int pp = m; pp >= 0; pp -= 2) {
-                const double c = lg[pp];
-                AI += c * Tm[k * kTmLd + pp];
-                E += c * Tm[k * kTmLd + NL + pp + 2];
-#pragma unroll
-                for (int o = 0; o < 5; ++o) {
-                    const int kk = k - 2 + o;
-                    if (kk >= 0) R0[o] += c * Tm[kk * kTmLd + NL + pp];
-                }
-#pragma unroll
-                for (int o = 0; o < 3; ++o) {
-                    const int kk = k - 1 + o;
-                    if (kk >= 0) C0[o] -= c * Tm[kk * kTmLd + NL + pp + 1];
-                }
+        if (!direct) {
+            float2 *dst = reinterpret_cast<float2 *>(a.nearbuf + (slot0 + s0) * kNearBlock);
+            for (int e = lane; e < npair * N * (kNearWeight / 2); e += 32) {
+                const int r = e / (kNearWeight / 2), w = e % (kNearWeight / 2);  // r: (pair, weight)
+                dst[(r / N) * (kNearBlock / 2) + (r % N) * (kNearWeight / 2) + w] =
+                    *reinterpret_cast<const float2 *>(s_rec + r * kNearStage + 2 * w);
             }
-            const double *al = s_bon, *be = s_bon + 8;
-            const double R1p = al[k + 1] * R0[4] + be[k + 1] * R0[2];                // R1_{k+1}
-            const double R1m = k > 0 ? al[k - 1] * R0[2] + be[k - 1] * R0[0] : 0.0;  // R1_{k-1}
-            const double R1 = al[k] * R0[3] + be[k] * R0[1];
-            const double R2 = al[k] * R1p + be[k] * R1m;
-            const double C1 = al[k] * C0[2] + be[k] * C0[0];
-            // theta = AI I + D X^T + t Y^T + p Z^T,  Q = theta t
-            double X[3], Y[3], Z[3], Q[3];
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                X[c] = R0[2] * D[c] + R1 * t[c] + C0[1] * p[c];
-                Y[c] = R1 * D[c] + R2 * t[c] + C1 * p[c];
-                Z[c] = C0[1] * D[c] + C1 * t[c] + E * p[c];
-            }
-#pragma unroll
-            for (int c = 0; c < 3; ++c) Q[c] = AI * t[c] + Dt * X[c] + tt * Y[c] + pt * Z[c];
-            if (m == 0) {
-                const double Xf = X[0] * f[0] + X[1] * f[1] + X[2] * f[2];
-                const double Yf = Y[0] * f[0] + Y[1] * f[1] + Y[2] * f[2];
-                const double Zf = Z[0] * f[0] + Z[1] * f[1] + Z[2] * f[2];
-#pragma unroll
-                for (int c = 0; c < 3; ++c) rhs[3 * k + c] += AI * f[c] + D[c] * Xf + t[c] * Yf + p[c] * Zf;
-                continue;
-            }
-            float *rec = blk + (m - 1) * kNearWeight;
-            if (k >= 1) {
-                // k = 1: D1 t Q^T; k >= 2: gamma_k (theta - E_k t Q^T); one formula
-                // g (AI' I + D X'^T + t W^T + p Z'^T) with the row's coefficients
-                const bool one = k == 1;
-                const double g = one ? D1 : s_bon[16 + k], ek = s_bon[24 + k];
-                const double ai = one ? 0.0 : AI;
-                double W[3];
-#pragma unroll
-                for (int c = 0; c < 3; ++c) W[c] = one ? Q[c] : Y[c] - ek * Q[c];
-#pragma unroll
-                for (int bb = 0; bb < 3; ++bb) {
-                    const double xb = one ? 0.0 : X[bb], zb = one ? 0.0 : Z[bb];
-#pragma unroll
-                    for (int aa = 0; aa < 3; ++aa)
-                        rec[bb * RB + 3 * (k - 1) + aa] =
-                            (float)(g * ((aa == bb ? ai : 0.0) + D[aa] * xb + t[aa] * W[bb] + p[aa] * zb));
-                }
-            }
-            if (PANELS && k <= 1) {
-                // P0: sv theta; P1: sw (theta - t Q^T)
-                const double sc = k == 0 ? sv : sw, kq = k == 0 ? 0.0 : 1.0;
-#pragma unroll
-                for (int bb = 0; bb < 3; ++bb)
-#pragma unroll
-                    for (int aa = 0; aa < 3; ++aa)
-                        rec[3 * RB + k * 9 + bb * 3 + aa] = (float)(
-                            sc * ((aa == bb ? AI : 0.0) + D[aa] * X[bb] + t[aa] * (Y[bb] - kq * Q[bb]) + p[aa] * Z[bb]));
-            }
-        }
-        __syncwarp();
-        if (!DIRECT) {
-            float4 *dst = reinterpret_cast<float4 *>(a.nearbuf + (int64_t)(slot0 + sidx) * kNearBlock);
-            const float4 *src = reinterpret_cast<const float4 *>(blk);
-            for (int e = lane; e < kNearBlock / 4; e += 32) dst[e] = src[e];
         } else {
-            for (int e = lane; e < N * kNearWeight; e += 32) {
-                const int mm = e / kNearWeight, r = e - mm * kNearWeight;
-                const float v = blk[e];
+            for (int e = lane; e < npair * N * kNearWeight; e += 32) {
+                const int pr = e / (N * kNearWeight), mm = e / kNearWeight - pr * N, r = e % kNearWeight;
+                const int64_t j = list[s0 + pr];
+                const float v = s_rec[pr * SM::PAIR + mm * kNearStage + r];
                 if (r < 3 * RB) {
                     const int col = 3 * mm + r / RB, rr = r % RB;
-                    const int64_t idx = ((int64_t)j * RB + col) * a.lda + (int64_t)i * RB + rr;
+                    const int64_t idx = (j * RB + col) * a.lda + (int64_t)i * RB + rr;
                     if (a.A16lo) {
                         split_store(v, a.A16 + idx, a.A16lo + idx);
                     } else {
@@ -1043,17 +1026,17 @@ __global__ void __launch_bounds__(kNearWarps * 32, RF_NEAR_MINB) near_pairs_kern
                     }
                 } else if (PANELS && r < 3 * RB + 18) {
                     const int e2 = r - 3 * RB, w = e2 / 9, rem = e2 - w * 9, bb = rem / 3, aa = rem - bb * 3;
-                    (w ? a.PW32 : a.PV32)[((int64_t)j * RB + 3 * mm + bb) * a.ldp + (int64_t)i * 3 + aa] = v;
+                    (w ? a.PW32 : a.PV32)[(j * RB + 3 * mm + bb) * a.ldp + (int64_t)i * 3 + aa] = v;
                 }
             }
         }
         __syncwarp();
     }
     __syncthreads();
-    for (int r = threadIdx.x; r < NRHS; r += blockDim.x) {
+    for (int r = tid; r < NRHS; r += kNearWarps * 32) {
         double s = 0.0;
-#pragma unroll
-        for (int w = 0; w < kNearWarps; ++w) s += s_wP[SM::TABLES + (size_t)w * SM::WARP + SM::X + SM::TM + SM::BLK + r];
+        for (int w = 0; w < kNearWarps * kTI; ++w)
+            s += (s_warp + (w / kTI) * SM::warp(LQ) + SM::region(LQ) + kTI * 6)[(w % kTI) * NRHS + r];
         a.near_contr[(int64_t)i * NRHS + r] = s;
     }
 }
@@ -1099,13 +1082,14 @@ cudaError_t launch_far_n(const SplitArgs &a, int far_chunks, cudaStream_t st) {
     return cudaGetLastError();
 }
 
-template <int N, bool PANELS, bool DIRECT>
-cudaError_t launch_near_n(const SplitArgs &a, cudaStream_t st) {
-    const size_t smem = NearSmem<N>::bytes();
-    auto kern = near_pairs_kernel<N, PANELS, DIRECT>;
+template <int N, bool PANELS>
+cudaError_t launch_near_n(const SplitArgs &a, bool direct, cudaStream_t st) {
+    const size_t smem = NearSmem<N>::bytes(a.LQ);
+    // tensor-core k-steps: 6 cover the usual 24 points
+    auto kern = a.LQ <= 24 ? near_pairs_kernel<N, PANELS, 6> : near_pairs_kernel<N, PANELS, kMaxLQ / 4>;
     cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (err != cudaSuccess) return err;
-    kern<<<a.M, kNearWarps * 32, smem, st>>>(a);
+    kern<<<a.M, kNearWarps * 32, smem, st>>>(a, direct);
     return cudaGetLastError();
 }
 
@@ -1174,10 +1158,8 @@ cudaError_t launch_split_far(const SplitArgs &a, int far_chunks, cudaStream_t st
 cudaError_t launch_split_near(const SplitArgs &a, bool direct, cudaStream_t st) {
     const bool panels = a.PV32 != nullptr;
     switch (a.N) {
-#define RF_NEAR_CASE(n)                                                                                    \
-    case n:                                                                                                \
-        if (panels) return direct ? launch_near_n<n, true, true>(a, st) : launch_near_n<n, true, false>(a, st); \
-        return direct ? launch_near_n<n, false, true>(a, st) : launch_near_n<n, false, false>(a, st);
+#define RF_NEAR_CASE(n) \
+    case n: return panels ? launch_near_n<n, true>(a, direct, st) : launch_near_n<n, false>(a, direct, st);
         RF_NEAR_CASE(1)
         RF_NEAR_CASE(2)
         RF_NEAR_CASE(3)
