@@ -8,13 +8,20 @@
 // step queued after the stop costs a few empty launches.  The inner solves of
 // the mixed-precision refinement and the FP64 and FP32 GMRES all run this way
 // (restart lengths up to kArnoldiMax; longer ones use the host-controlled
-// solver; small FP64 systems run in one kernel, gmres_small.cu).  What bounds a small system is the number of dependent launches: a
-// step is the product's two kernels, three orthogonalisation passes and one
-// scaling, where the host-controlled solver takes j + 5 launches, a copy and
-// a wait of the host.  Whole time steps,
-// FP64: M = 100 (18 iterations) 1.70 -> 0.96 ms, M = 333 (N = 3) 2.24 -> 1.51
-// ms, M = 1000 (products of 0.28 ms) 13.9 -> 12.8 ms; FP32 M = 1000 6.04 ->
-// 5.57 ms.
+// solver; small FP64 systems run in one kernel, gmres_small.cu).  What bounds a
+// small system is the number of dependent launches: a step is the product's two
+// kernels, three orthogonalisation passes and one scaling, where the
+// host-controlled solver takes j + 5 launches, a copy and a wait of the host.
+// Whole time steps, FP64: M = 1000 (products of 0.28 ms) 13.9 -> 12.8 ms; FP32
+// M = 1000 6.04 -> 5.57 ms.
+//
+// Restarts: the residual of the updated x is V_{0..m} Q^T (0, .., 0, g_m), Q the
+// cycle's rotations, to rounding (A V = V H holds to rounding), so a cycle ends
+// without the product b - A x that the reference makes (dGMRES.f, one product in
+// m + 1; FP64 M = 1000, 21 iterations: 25 -> 23 products of 0.28 ms).  The
+// solution is still accepted only on the true residual; after one that was not
+// within the tolerance, where the difference of the two residuals may be what
+// is left, the solve's later restarts make the product.
 //
 // Orthogonalisation: classical Gram-Schmidt applied twice (CGS2), fused into
 // three passes over the basis: (1) h1 = V^T w; (2) w -= V h1, h2 = V^T w;
@@ -108,12 +115,31 @@ __device__ __forceinline__ void rot_d(double &x, double &y, double c, double s) 
     x = t;
 }
 
+// |r|.  kind = kStartBasis: w holds the unscaled next basis vector of a finished
+// cycle of m steps and becomes the residual of the updated x, r = w.
 template <typename T>
-__global__ void __launch_bounds__(kThreads) start_kernel(int64_t n, const T *__restrict__ r, ArnoldiCtrl *c,
-                                                         double tol, int iter_max, int kind, double *part,
-                                                         unsigned int *counter, ArnoldiStat *stat) {
+__global__ void __launch_bounds__(kThreads) start_kernel(int64_t n, const T *r, T *w, const T *V, int m, ArnoldiCtrl *c, double tol, int iter_max, int kind,
+                                                         double *part, unsigned int *counter, ArnoldiStat *stat) {
+    __shared__ double ts[KM + 1];
+    if (kind == kStartBasis) {
+        if (threadIdx.x == 0) {
+            double t = c->g[m];
+            for (int q = m - 1; q >= 0; --q) {
+                ts[q + 1] = c->cs[q] * t;
+                t *= -c->sn[q];
+            }
+            ts[0] = t;
+            ts[m] /= c->hnext;
+        }
+        __syncthreads();
+    }
     double v[1] = {0.0};
     for (int64_t e = (int64_t)blockIdx.x * kThreads + threadIdx.x; e < n; e += (int64_t)gridDim.x * kThreads) {
+        if (kind == kStartBasis) {
+            double s = ts[m] * (double)w[e];
+            for (int q = 0; q < m; ++q) s += ts[q] * (double)V[(int64_t)q * n + e];
+            w[e] = (T)s;
+        }
         const double x = (double)r[e];
         v[0] += x * x;
     }
@@ -313,11 +339,11 @@ __global__ void vy_kernel(int64_t n, const T *__restrict__ V, const ArnoldiCtrl 
 }  // namespace
 
 template <typename T>
-cudaError_t launch_arnoldi_start(int64_t n, const T *r, T *V0, ArnoldiCtrl *c, double tol, int iter_max,
+cudaError_t launch_arnoldi_start(int64_t n, const T *r, T *w, T *V0, int m, ArnoldiCtrl *c, double tol, int iter_max,
                                  ArnoldiStart kind, double *part, unsigned int *counter, int max_blocks,
                                  ArnoldiStat *stat, cudaStream_t st) {
     const int nb = blocks_for(n, max_blocks);
-    start_kernel<T><<<nb, kThreads, 0, st>>>(n, r, c, tol, iter_max, kind, part, counter, stat);
+    start_kernel<T><<<nb, kThreads, 0, st>>>(n, r, w, V0, m, c, tol, iter_max, kind, part, counter, stat);
     scale_next_kernel<T><<<nb, kThreads, 0, st>>>(n, r, V0, c, 0);
     return cudaGetLastError();
 }
@@ -349,12 +375,12 @@ cudaError_t launch_arnoldi_combine(int64_t n, const T *V, ArnoldiCtrl *c, T *u, 
     return cudaGetLastError();
 }
 
-template cudaError_t launch_arnoldi_start<float>(int64_t, const float *, float *, ArnoldiCtrl *, double, int,
-                                                 ArnoldiStart, double *, unsigned int *, int, ArnoldiStat *,
-                                                 cudaStream_t);
-template cudaError_t launch_arnoldi_start<double>(int64_t, const double *, double *, ArnoldiCtrl *, double, int,
-                                                  ArnoldiStart, double *, unsigned int *, int, ArnoldiStat *,
-                                                  cudaStream_t);
+template cudaError_t launch_arnoldi_start<float>(int64_t, const float *, float *, float *, int, ArnoldiCtrl *,
+                                                 double, int, ArnoldiStart, double *, unsigned int *, int,
+                                                 ArnoldiStat *, cudaStream_t);
+template cudaError_t launch_arnoldi_start<double>(int64_t, const double *, double *, double *, int, ArnoldiCtrl *,
+                                                  double, int, ArnoldiStart, double *, unsigned int *, int,
+                                                  ArnoldiStat *, cudaStream_t);
 template cudaError_t launch_arnoldi_orthogonalize<float>(int64_t, float *, float *, int, int, ArnoldiCtrl *,
                                                          ArnoldiStat *, double *, unsigned int *, int, cudaStream_t);
 template cudaError_t launch_arnoldi_orthogonalize<double>(int64_t, double *, double *, int, int, ArnoldiCtrl *,

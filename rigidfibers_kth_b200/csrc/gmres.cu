@@ -100,7 +100,7 @@ cudaError_t Gmres<VT>::solve_device(const StopOp &A, const StopOp *P, const VT *
     volatile ArnoldiStat *hs = hstat_;
     auto start = [&](const VT *r, ArnoldiStart kind) {
         res->launches += 2;
-        return launch_arnoldi_start<VT>(n_, r, V_, ctrl_, tol, iterMax, kind, cpart_, rb_.counter, rb_.max_blocks,
+        return launch_arnoldi_start<VT>(n_, r, w_, V_, m, ctrl_, tol, iterMax, kind, cpart_, rb_.counter, rb_.max_blocks,
                                         dstat_ + kArnoldiMax, st_);
     };
     auto resid = [&](const VT *xv) -> cudaError_t {  // w_ = b - A xv
@@ -118,6 +118,7 @@ cudaError_t Gmres<VT>::solve_device(const StopOp &A, const StopOp *P, const VT *
         RF_TRY(start(w_, kStartFrom));
     }
     int last_stop = 0;
+    bool check_failed = false;  // an estimate within the tolerance whose true residual was not
     for (;;) {
         // The start of a cycle may already stop the solve (zero or non-finite
         // residual).  Its outcome is read after the first step's event: steps
@@ -215,13 +216,19 @@ cudaError_t Gmres<VT>::solve_device(const StopOp &A, const StopOp *P, const VT *
             }
             // not there yet: this cycle goes on with step done + 1 (its basis
             // vector is in place), or restarts if that was its last step
+            check_failed = true;
             RF_TRY(cudaMemsetAsync(&ctrl_->stop, 0, sizeof(int), st_));
             j = done + 1;
             if (j == m) RF_TRY(cudaMemcpyAsync(x, xcur_, sizeof(VT) * n_, cudaMemcpyDeviceToDevice, st_));
         }
-        // restart from the residual of the updated x
-        RF_TRY(resid(x));
-        RF_TRY(start(w_, kStartFrom));
+        // restart from the residual of the updated x, without a product where
+        // the cycle's basis may give it (arnoldi.cu)
+        if (check_failed) {
+            RF_TRY(resid(x));
+            RF_TRY(start(w_, kStartFrom));
+        } else {
+            RF_TRY(start(w_, kStartBasis));
+        }
     }
 }
 

@@ -46,7 +46,7 @@ struct Shared {
     double w[kSmallRows], x[kSmallRows], xcur[kSmallRows], b[kSmallRows];
     double red[kThreads / 16][kSmallRows + 1];     // slices of a row's partial sums
     double h1[KM], h2[KM];
-    double H[KM][KM], g[KM + 1], cs[KM], sn[KM], y[KM];
+    double H[KM][KM], g[KM + 1], cs[KM], sn[KM], y[KM + 1];
     double sum[2];
     int failed;
 };
@@ -248,6 +248,7 @@ struct Solver {
         double beta = sqrt(s.sum[0]);
         if (!isfinite(beta)) return leave(kSmallNaN);
         if (beta == 0.0) return leave(kSmallOk);
+        bool check_failed = false;  // an estimate within the tolerance whose true residual was not
         for (;;) {
             double norm = beta;  // of the vector in a.w
             if (threadIdx.x <= KM) s.g[threadIdx.x] = threadIdx.x == 0 ? beta : 0.0;
@@ -317,17 +318,38 @@ struct Solver {
                 }
                 for (int r = threadIdx.x; r < rows; r += kThreads) s.w[r] = j + 1 < KM ? s.V[KM - 1][r] : 0.0;
                 __syncthreads();
+                check_failed = true;
             }
-            // restart from the residual of the updated x
-            if (!stopped) {
-                combine(a.m);
+            // restart from the residual of the updated x, without a product
+            // where the cycle's basis may give it (arnoldi.cu)
+            if (!stopped) combine(a.m);
+            for (int r = threadIdx.x; r < rows; r += kThreads) s.x[r] = s.xcur[r];
+            if (check_failed) {
                 publish(a.xcur, s.xcur);
                 if (!barrier()) return leave(kSmallTimeout);
+                ++st.matvecs;
+                if (!residual(a.xcur, &beta)) return leave(kSmallTimeout);
+            } else {
+                if (threadIdx.x == 0) {
+                    double t = s.g[a.m];
+                    for (int q = a.m - 1; q >= 0; --q) {
+                        s.y[q + 1] = s.cs[q] * t;
+                        t *= -s.sn[q];
+                    }
+                    s.y[0] = t;
+                    s.y[a.m] /= norm;
+                }
+                __syncthreads();
+                for (int r = threadIdx.x; r < rows; r += kThreads) {
+                    double t = s.y[a.m] * s.w[r];
+                    for (int q = 0; q < a.m; ++q) t += s.y[q] * s.V[q][r];
+                    s.w[r] = t;
+                    a.w[r0 + r] = t;
+                }
+                __syncthreads();
+                if (!dots(1, 0, [&](int, int r) { return s.w[r] * s.w[r]; }, s.sum)) return leave(kSmallTimeout);
+                beta = sqrt(s.sum[0]);
             }
-            for (int r = threadIdx.x; r < rows; r += kThreads) s.x[r] = s.xcur[r];
-            __syncthreads();
-            ++st.matvecs;
-            if (!residual(a.xcur, &beta)) return leave(kSmallTimeout);
             if (!isfinite(beta)) return leave(kSmallNaN);
             if (beta == 0.0) {
                 publish(a.x, s.x);

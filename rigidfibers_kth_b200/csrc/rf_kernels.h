@@ -300,8 +300,10 @@ constexpr int kStopBudget = 2;    // step budget spent
 constexpr int kStopNaN = 3;       // non-finite value
 constexpr int kStopZeroRhs = 4;   // |b| = 0 at a cycle's start
 // What a cycle starts from: the solve's right-hand side (records |b|, the
-// tolerance and the budget) or the residual of a current iterate.
-enum ArnoldiStart { kStartSolve, kStartFrom };
+// tolerance and the budget), the residual of a current iterate, or the residual
+// that the last cycle's basis gives (its m steps done, stop = 0; w = the unscaled
+// vector V_m on entry, the residual on return).
+enum ArnoldiStart { kStartSolve, kStartFrom, kStartBasis };
 // One step's outcome as the host sees it (host-mapped memory written by the device).
 struct ArnoldiStat {
     int stop;
@@ -311,9 +313,9 @@ struct ArnoldiStat {
 // Start of a cycle: beta = |r| (r the cycle's residual); g = (beta, 0, ...),
 // k = 0, stop = 0 (or the outcome of a zero or non-finite residual), written
 // to *stat (host-mapped) too; kStartSolve also sets bn = beta, itn = 0 and the
-// tolerance and budget; then V_0 = r / beta.
+// tolerance and budget; then V_0 = r / beta.  w, m: for kStartBasis, where r = w.
 template <typename T>
-cudaError_t launch_arnoldi_start(int64_t n, const T *r, T *V0, ArnoldiCtrl *c, double tol, int iter_max,
+cudaError_t launch_arnoldi_start(int64_t n, const T *r, T *w, T *V0, int m, ArnoldiCtrl *c, double tol, int iter_max,
                                  ArnoldiStart kind, double *part, unsigned int *counter, int max_blocks,
                                  ArnoldiStat *stat, cudaStream_t st);
 // Step j after w = A z: two classical Gram-Schmidt passes against V_0..V_j

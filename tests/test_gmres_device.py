@@ -101,3 +101,22 @@ def test_one_rank_communicator_above_the_single_kernel_solver():
             out.append(s.state() + s.velocities() + (s.coeffs(), s.rhs()))
     for a, b in zip(*out):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("restart", [1, 2, 5, 10, 16])
+@pytest.mark.parametrize("passes", [False, True])
+def test_restarts_without_a_product(restart, passes):
+    """The residual of a restart comes from the cycle's basis: the iterates stay
+    the oracle's, which makes the product, over many short cycles, in the
+    single-kernel solver and in launched passes; products are made for the start
+    and for the accepted solution only."""
+    sim, A, b = system(37, gmres_restart=restart, gmres_tol=1e-10, gmres_max_iters=600)
+    with sim:
+        sim.gemv_timer(passes)
+        assert sim.solve_system() == 0
+        x, st = sim.coeffs(), sim.solve_stats()
+    x_o, info, iters, _ = rfo.solve_gmres(A, b, restart=restart, max_iters=600, tol=1e-10)
+    assert info == 0 and st["iterations"] == iters and iters > restart
+    assert st["matvecs"] == iters + 2
+    assert np.linalg.norm(b - A @ x) <= 1e-10 * np.linalg.norm(b) * (1 + 1e-4)
+    assert np.abs(x - x_o).max() <= 1e-10 * np.abs(x_o).max()
