@@ -65,3 +65,25 @@ def test_ragged_sizes(M, N, NoQI, reuse):
     V_o, W_o = rfo.velocities(p, pos, ori, x)
     assert np.abs(V - V_o).max() <= 1e-10 * np.abs(V_o).max()
     assert np.abs(W - W_o).max() <= 1e-10 * max(np.abs(W_o).max(), np.abs(V_o).max())
+
+
+@pytest.mark.parametrize("N,NoQI", [(1, 3), (3, 8), (5, 8), (8, 8)])
+@pytest.mark.parametrize("gap", [0.3, 0.05, 0.01])
+@pytest.mark.parametrize("eps", [1e-3, 1e-2])
+def test_numeric_integral_of_close_pairs(N, NoQI, gap, eps):
+    """The numeric inner integral of two crossing fibers.  Both sides round the
+    positions (a few units of |x| <= 2, relative to the gap) under a fifth power
+    of the distance: 5 x 2 units, four times for the sums."""
+    rng = np.random.default_rng(int(1000 * gap) + N)
+    t = unit(rng.normal(size=(2, 3)))
+    s = rng.uniform(-0.9, 0.9, 2)
+    pos = np.array([[0.0, 0.0, 0.0], gap * unit(np.cross(t[0], t[1])) + s[0] * t[0] - s[1] * t[1]])
+    p = rf.FiberParams(slenderness=eps, num_terms_in_force_expansion=N, num_quadrature_intervals=NoQI,
+                       use_analytical_integration=0)
+    with rf.Simulation(rf.Configuration(p, pos, t)) as sim:
+        sim.assemble_system()
+        A, b = sim.matrix(), sim.rhs()
+    A_o, b_o = rfo.assemble_system(rfo.make_params(2, N=N, NoQI=NoQI, eps=eps, analytic=False), pos, t)
+    tol = 40 * 2.0 ** -52 * (1 + 2 / gap)
+    assert np.abs(A - A_o).max() <= tol * np.abs(A_o).max()
+    assert np.abs(b - b_o).max() <= tol * np.abs(b_o).max()
