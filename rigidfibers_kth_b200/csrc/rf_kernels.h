@@ -349,8 +349,7 @@ struct SmallGmresArgs {
     unsigned *barrier;        // device word
     SmallGmresStat *stat;     // device
     // set by the launcher
-    int tiles, splits, cols;
-    double *part, *dots, *w, *xcur;
+    double *sums, *w, *xcur;
 };
 bool gmres_small_supported(int64_t n, int m, int sm_count);
 int64_t gmres_small_work(int64_t n, int sm_count);   // doubles of `work`

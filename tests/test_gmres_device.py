@@ -120,3 +120,17 @@ def test_restarts_without_a_product(restart, passes):
     assert st["matvecs"] == iters + 2
     assert np.linalg.norm(b - A @ x) <= 1e-10 * np.linalg.norm(b) * (1 + 1e-4)
     assert np.abs(x - x_o).max() <= 1e-10 * np.abs(x_o).max()
+
+
+# rows per CTA of the single-kernel solver that are not whole groups of eight,
+# with four, two and one columns in flight per warp, even and odd sizes; M = 1 and
+# 2 end in a breakdown, where |w - V h2| is not |w|^2 - |h2|^2
+@pytest.mark.parametrize("M,N,restart", [(1, 5, 10), (2, 5, 10), (101, 5, 10), (193, 5, 16), (333, 3, 5), (345, 5, 10)])
+def test_single_kernel_solver_row_shapes(M, N, restart):
+    sim, A, b = system(M, num_terms_in_force_expansion=N, gmres_restart=restart, gmres_tol=1e-12, gmres_max_iters=300)
+    with sim:
+        assert sim.solve_system() == 0
+        x, st = sim.coeffs(), sim.solve_stats()
+    # the true residual was accepted; numpy's differs by the rounding of n products
+    assert np.linalg.norm(b - A @ x) <= (1e-12 + 3 * len(b) * 2.0 ** -53) * np.linalg.norm(b)
+    assert abs(st["residual"] - np.linalg.norm(b - A @ x) / np.linalg.norm(b)) <= 3 * len(b) * 2.0 ** -53
