@@ -2,7 +2,7 @@
 // reference Fortran solver (fortran/dGMRES.f:491-1495 as configured by
 // fortran/coeffs_and_vels.f90:446-500): modified Gram-Schmidt, Givens
 // rotations on the Hessenberg matrix, the true residual recomputed at each
-// restart, and the stopping rule "Arnoldi estimate <= tol, then true
+// restart (solve_device: from the basis, arnoldi.cu), and the stopping rule "Arnoldi estimate <= tol, then true
 // residual <= tol" on ||b - A x|| / ||b||.  Right preconditioning z = P v is
 // optional (the residual keeps its meaning).  Krylov vectors live on the
 // device in VT (double or float); the Hessenberg matrix, rotations and the

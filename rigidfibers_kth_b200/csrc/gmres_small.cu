@@ -27,7 +27,7 @@
 // long sets an error and the CTAs leave.
 //
 // Device-controlled passes -> this kernel, a step to 1e-10: n = 1500 31 -> 12.5
-// us, n = 3000 38 -> 17 us, n = 4500 (162 MB, from memory) 58 -> 34 us.
+// us, n = 3000 44 -> 17 us, n = 4500 (162 MB, from memory) 58 -> 34 us.
 // Systems up to kSmallMaxN = 8192: there the product of 537 MB takes 80 of the
 // 90 us a step costs here, and the passes' launches hide behind it from about
 // there on; a CTA's rows (kSmallRows = 64 on each SM) end at 9472.

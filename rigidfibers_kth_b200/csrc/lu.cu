@@ -12,7 +12,8 @@
 //   lu_panel_update_kernel  the W columns' update of the rest of the panel,
 //                           over the whole GPU;
 //   lu_trsm_kernel          the panel's row swaps on the trailing columns and
-//                           U12 = L11^-1 A12, one thread per column;
+//                           U12 = L11^-1 A12 in shared memory, block by block
+//                           on the FP64 tensor cores;
 //   lu_gemm_kernel          A22 -= L21 U12, the rank-128 trailing update on
 //                           the FP64 tensor cores: most of the 2/3 n^3 flops;
 //   lu_back_kernel          back substitution, 128 rows at a time.
