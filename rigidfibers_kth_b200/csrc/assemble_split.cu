@@ -68,85 +68,6 @@ __host__ __device__ constexpr int vrows(int N, int p) { return p <= N ? N + 3 : 
 __host__ __device__ constexpr double bonnet_a(int k) { return (k + 1.0) / (2.0 * k + 1.0); }
 __host__ __device__ constexpr double bonnet_b(int k) { return k / (2.0 * k + 1.0); }
 
-// Scalar coefficient sets of source weight m from the projections
-// U(p, k) = <u_p>_k and V(p, k) = <v_p>_k.
-template <typename T, int N>
-struct LegSets {
-    T AI[N + 1], R0[N + 3], R1[N + 2], R2[N + 1], C0[N + 2], C1[N + 1], E[N + 1];
-};
-
-template <typename T, int N, int m, typename UF, typename VF>
-__device__ __forceinline__ void leg_sets(const UF &U, const VF &V, LegSets<T, N> &o) {
-    const T sc = (T)leg_scale(m);
-#pragma unroll
-    for (int k = 0; k <= N; ++k) {
-        T s = 0;
-#pragma unroll
-        for (int p = m; p >= 0; --p)
-            if (leg_coef(m, p) != 0) s += (T)leg_coef(m, p) * U(p, k);
-        o.AI[k] = sc * s;
-    }
-#pragma unroll
-    for (int k = 0; k <= N + 2; ++k) {
-        T s = 0;
-#pragma unroll
-        for (int p = m; p >= 0; --p)
-            if (leg_coef(m, p) != 0) s += (T)leg_coef(m, p) * V(p, k);
-        o.R0[k] = sc * s;
-    }
-#pragma unroll
-    for (int k = 0; k <= N + 1; ++k) {
-        T s = 0;
-#pragma unroll
-        for (int p = m; p >= 0; --p)
-            if (leg_coef(m, p) != 0) s += (T)leg_coef(m, p) * V(p + 1, k);
-        o.C0[k] = -sc * s;
-    }
-#pragma unroll
-    for (int k = 0; k <= N; ++k) {
-        T s = 0;
-#pragma unroll
-        for (int p = m; p >= 0; --p)
-            if (leg_coef(m, p) != 0) s += (T)leg_coef(m, p) * V(p + 2, k);
-        o.E[k] = sc * s;
-    }
-#pragma unroll
-    for (int k = 0; k <= N + 1; ++k)
-        o.R1[k] = (T)bonnet_a(k) * o.R0[k + 1] + (k > 0 ? (T)bonnet_b(k) * o.R0[k > 0 ? k - 1 : 0] : (T)0);
-#pragma unroll
-    for (int k = 0; k <= N; ++k) {
-        o.R2[k] = (T)bonnet_a(k) * o.R1[k + 1] + (k > 0 ? (T)bonnet_b(k) * o.R1[k > 0 ? k - 1 : 0] : (T)0);
-        o.C1[k] = (T)bonnet_a(k) * o.C0[k + 1] + (k > 0 ? (T)bonnet_b(k) * o.C0[k > 0 ? k - 1 : 0] : (T)0);
-    }
-}
-
-// The seven pair tensors, packed 11,22,33,12,13,23 (identity implicit).
-template <typename T>
-struct PairTensors {
-    T DD[6], DT[6], TT[6], PD[6], PT[6], PP[6];
-    __device__ __forceinline__ void set(const T *D, const T *t, const T *p) {
-        const int ia[6] = {0, 1, 2, 0, 0, 1}, ib[6] = {0, 1, 2, 1, 2, 2};
-#pragma unroll
-        for (int c = 0; c < 6; ++c) {
-            const int x = ia[c], y = ib[c];
-            DD[c] = D[x] * D[y];
-            DT[c] = D[x] * t[y] + t[x] * D[y];
-            TT[c] = t[x] * t[y];
-            PD[c] = p[x] * D[y] + D[x] * p[y];
-            PT[c] = p[x] * t[y] + t[x] * p[y];
-            PP[c] = p[x] * p[y];
-        }
-    }
-    // theta for projection row k of the sets
-    template <int N>
-    __device__ __forceinline__ void theta(const LegSets<T, N> &s, int k, T *th) const {
-#pragma unroll
-        for (int c = 0; c < 6; ++c)
-            th[c] = (c < 3 ? s.AI[k] : (T)0) + s.R0[k] * DD[c] + s.R1[k] * DT[c] + s.R2[k] * TT[c] +
-                    s.C0[k] * PD[c] + s.C1[k] * PT[c] + s.E[k] * PP[c];
-    }
-};
-
 // FP64 moments for the near pairs of the mixed path: the reference formulas
 // (Int_analytical.f90:96-207) with ordinary (contracted) arithmetic and the
 // loop-constant divisions folded into reciprocals.

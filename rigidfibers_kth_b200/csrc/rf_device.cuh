@@ -550,30 +550,6 @@ struct GStore<T, N, N + 1> {
     __device__ __forceinline__ static void run(const T *, const T *, const T *, const Outer<T> &, T, double *, int) {}
 };
 
-// u = sum_m G_m f_m without forming G_m:
-// G f = cI f + R0 (cRR R0.f + cPR pb.f) + pb (cPR R0.f + cPP pb.f)
-template <typename T, int N, int m = 0>
-struct GForce {
-    __device__ __forceinline__ static void run(const T *I, const T *J, const T *S, T r0x, T r0y, T r0z, T px,
-                                               T py, T pz, T eps2, const T (*f)[3], T *u) {
-        T cI, cRR, cPR, cPP;
-        g_coeffs<T, m>(I, J, S, eps2, cI, cRR, cPR, cPP);
-        const T rf = r0x * f[m][0] + r0y * f[m][1] + r0z * f[m][2];
-        const T pf = px * f[m][0] + py * f[m][1] + pz * f[m][2];
-        const T aR = cRR * rf + cPR * pf;
-        const T aP = cPR * rf + cPP * pf;
-        u[0] += cI * f[m][0] + aR * r0x + aP * px;
-        u[1] += cI * f[m][1] + aR * r0y + aP * py;
-        u[2] += cI * f[m][2] + aR * r0z + aP * pz;
-        GForce<T, N, m + 1>::run(I, J, S, r0x, r0y, r0z, px, py, pz, eps2, f, u);
-    }
-};
-template <typename T, int N>
-struct GForce<T, N, N + 1> {
-    __device__ __forceinline__ static void run(const T *, const T *, const T *, T, T, T, T, T, T, T,
-                                               const T (*)[3], T *) {}
-};
-
 // The analytic inner integral for all weights, stored to shared memory.
 template <int N>
 __device__ __forceinline__ void inner_analytic_store_fp64(double r0x, double r0y, double r0z, double px, double py,
@@ -593,18 +569,6 @@ __device__ __forceinline__ void inner_analytic_store_fp32(float r0x, float r0y, 
     moments_fp32<N>(Geom32(r0x, r0y, r0z, px, py, pz), I, J, S);
     const Outer<float> o(r0x, r0y, r0z, px, py, pz);
     GStore<float, N>::run(I, J, S, o, eps2, dst, ld);
-}
-
-// sum_m G_m f_m at one target point (FP64): the velocity integrand
-// (G_compute_GQ_f_kg, Int_analytical.f90:772-850)
-template <int N>
-__device__ __forceinline__ void inner_analytic_force_fp64(double r0x, double r0y, double r0z, double px, double py,
-                                                          double pz, double eps2, const double (*f)[3], double *u) {
-    double I[N + 3], J[N + 3], S[N + 3];
-    const double b = fmul(-2.0, fadd(fadd(fmul(px, r0x), fmul(py, r0y)), fmul(pz, r0z)));
-    const double c = fadd(fadd(fmul(r0x, r0x), fmul(r0y, r0y)), fmul(r0z, r0z));
-    moments_fp64<N>(b, c, I, J, S);
-    GForce<double, N>::run(I, J, S, r0x, r0y, r0z, px, py, pz, eps2, f, u);
 }
 
 // Numeric inner integral (quadrature.f90:100-164): 3-point Gauss on each
