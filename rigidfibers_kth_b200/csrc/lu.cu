@@ -97,12 +97,17 @@ __device__ __forceinline__ void load_row(double (&v)[W], const double *s) {
     if (W % 2) v[W - 1] = s[W - 1];
 }
 
+// far from both ends of the range (and not zero, infinite or NaN): rcp_pos holds
+// its bound and div_by's products and remainder are normal numbers
+__device__ __forceinline__ bool mid_range(double v) {
+    const double m = fabs(v);
+    return m > 1e-290 && m < 1e290;
+}
+
 // 1/d as the division gives it, without its branches where d is far from the
 // ends of the range
 __device__ __forceinline__ double pivot_reciprocal(double d) {
-    const double m = fabs(d);
-    if (m > 1e-290 && m < 1e290) return div_by(1.0, d, copysign(rcp_pos(m), d));
-    return 1.0 / d;
+    return mid_range(d) ? div_by(1.0, d, copysign(rcp_pos(fabs(d)), d)) : 1.0 / d;
 }
 
 // The interchanges of slots 0..w-1 with slots to[0..w-1] (to[t] >= t; slot
@@ -608,8 +613,11 @@ __global__ void __launch_bounds__(kGThreads, 2) lu_gemm_kernel(const double *__r
 
 // Back substitution, rows [k, k + nb): the triangle in shared memory, by blocks
 // of 32 rows from the last (one warp, the block's rows in its lanes, x_p
-// broadcast by shuffles, quotients from each lane's reciprocal), each solved
-// block taken off the rows above it by all warps.
+// broadcast by shuffles, quotients from each lane's reciprocal where operands
+// and quotient are far from the ends of the range, else by the division: a
+// subnormal or huge pivot has no usable reciprocal, and zero, overflowing and
+// subnormal quotients need the division's own rounding), each solved block
+// taken off the rows above it by all warps.
 constexpr int kBackThreads = 512;
 constexpr int kBackLd = kLuNb + 1;
 __global__ void __launch_bounds__(kBackThreads) lu_back_diag_kernel(const double *__restrict__ A, int64_t lda,
@@ -629,10 +637,11 @@ __global__ void __launch_bounds__(kBackThreads) lu_back_diag_kernel(const double
         const int bn = min(32, nb - b);
         if (tid < 32) {
             double xi = lane < bn ? s_x[b + lane] : 0.0;
-            const double d = lane < bn ? s_u[(b + lane) * kBackLd + b + lane] : 1.0, rd = rcp_pos(fabs(d));
+            const double d = lane < bn ? s_u[(b + lane) * kBackLd + b + lane] : 1.0;
+            const double rd = mid_range(d) ? copysign(rcp_pos(fabs(d)), d) : 0.0;  // 0: no quotient is in range
             for (int p = bn - 1; p >= 0; --p) {
                 const double u = lane < p ? s_u[(b + p) * kBackLd + b + lane] : 0.0;
-                if (lane == p) xi = div_by(xi, d, copysign(rd, d));
+                if (lane == p) xi = mid_range(xi) && mid_range(xi * rd) ? div_by(xi, d, rd) : xi / d;
                 const double xp = __shfl_sync(0xffffffffu, xi, p);
                 if (lane < p) xi = fma(-u, xp, xi);
             }
