@@ -47,6 +47,7 @@ constexpr int kPanelThreads = 256;
 constexpr int kPanelWarps = kPanelThreads / 32;
 constexpr int kMaxCluster = 16;
 constexpr unsigned kNoRow = 0xffffffffu;
+constexpr double kMinNormal = 2.2250738585072014e-308, kSubScale = 18446744073709551616.0;  // 2^-1022, 2^64
 
 // A pivot candidate: |value| as an ordered integer (high and low word; none and
 // NaN: 0 with row kNoRow, but a NaN on the diagonal stands as a zero, so that a
@@ -97,17 +98,13 @@ __device__ __forceinline__ void load_row(double (&v)[W], const double *s) {
     if (W % 2) v[W - 1] = s[W - 1];
 }
 
-// far from both ends of the range (and not zero, infinite or NaN): rcp_pos holds
-// its bound and div_by's products and remainder are normal numbers
+// far from both ends of the range, 2^-959 <= |v| < 2^960 (and so not zero,
+// infinite or NaN): rcp_pos holds its bound and div_by's products and remainder
+// are normal numbers.  On the exponent: two integer operations, where FP64
+// comparisons stood in the serial chain of the back substitution.
 __device__ __forceinline__ bool mid_range(double v) {
-    const double m = fabs(v);
-    return m > 1e-290 && m < 1e290;
-}
-
-// 1/d as the division gives it, without its branches where d is far from the
-// ends of the range
-__device__ __forceinline__ double pivot_reciprocal(double d) {
-    return mid_range(d) ? div_by(1.0, d, copysign(rcp_pos(fabs(d)), d)) : 1.0 / d;
+    constexpr unsigned lo = 64u << 20, hi = 1983u << 20;
+    return ((unsigned)__double2hiint(v) & 0x7fffffffu) - lo < hi - lo;
 }
 
 // The interchanges of slots 0..w-1 with slots to[0..w-1] (to[t] >= t; slot
@@ -261,7 +258,7 @@ __global__ void __launch_bounds__(kPanelThreads) lu_panel_kernel(double *A, int6
             piv[col] = (int)c.row;
             if (d == 0.0 && *info == 0) *info = (int)(col + 1);
         }
-        const double inv = d != 0.0 ? pivot_reciprocal(d) : 1.0;  // a zero pivot leaves its column (dgetf2)
+        double inv = div_by(1.0, d, copysign(rcp_pos(fabs(d)), d));  // 1/d as the division gives it, where d is in mid range
         if (p != col) {
 #pragma unroll
             for (int u = 0; u < R; ++u) {
@@ -269,6 +266,16 @@ __global__ void __launch_bounds__(kPanelThreads) lu_panel_kernel(double *A, int6
                 if (r == p) load_row<W>(v[u], s_diag[buf]);
                 else if (r == col) load_row<W>(v[u], s_full[buf][slot]);  // the first CTA's
             }
+        }
+        if (!mid_range(d)) {
+            // a zero pivot leaves its column (dgetf2).  A subnormal one's reciprocal
+            // overflows: pivot and column are scaled up, which is exact (no entry
+            // is larger than the pivot); dgetf2 divides there.
+            const double up = fabs(d) < kMinNormal ? kSubScale : 1.0;
+            inv = d != 0.0 ? 1.0 / (d * up) : 1.0;
+#pragma unroll
+            for (int u = 0; u < R; ++u)
+                if (s0 + g + u * stride > col) v[u][0] *= up;
         }
         double nx[R];  // minus the multiplier; rows above keep their values
 #pragma unroll
@@ -613,11 +620,12 @@ __global__ void __launch_bounds__(kGThreads, 2) lu_gemm_kernel(const double *__r
 
 // Back substitution, rows [k, k + nb): the triangle in shared memory, by blocks
 // of 32 rows from the last (one warp, the block's rows in its lanes, x_p
-// broadcast by shuffles, quotients from each lane's reciprocal where operands
-// and quotient are far from the ends of the range, else by the division: a
-// subnormal or huge pivot has no usable reciprocal, and zero, overflowing and
-// subnormal quotients need the division's own rounding), each solved block
-// taken off the rows above it by all warps.
+// broadcast by shuffles), each solved block taken off the rows above it by all
+// warps.  Quotients come from each lane's reciprocal; a block in which a pivot,
+// an operand or a quotient is zero, not finite or near the ends of the range is
+// solved again with divisions (a subnormal or huge pivot has no usable
+// reciprocal; overflow and underflow need the division's own rounding).  The
+// choice per quotient instead cost 50 ns a row, 0.8 of 127 ms at n = 15000.
 constexpr int kBackThreads = 512;
 constexpr int kBackLd = kLuNb + 1;
 __global__ void __launch_bounds__(kBackThreads) lu_back_diag_kernel(const double *__restrict__ A, int64_t lda,
@@ -636,15 +644,25 @@ __global__ void __launch_bounds__(kBackThreads) lu_back_diag_kernel(const double
     for (int b = (nb - 1) / 32 * 32; b >= 0; b -= 32) {
         const int bn = min(32, nb - b);
         if (tid < 32) {
-            double xi = lane < bn ? s_x[b + lane] : 0.0;
-            const double d = lane < bn ? s_u[(b + lane) * kBackLd + b + lane] : 1.0;
-            const double rd = mid_range(d) ? copysign(rcp_pos(fabs(d)), d) : 0.0;  // 0: no quotient is in range
-            for (int p = bn - 1; p >= 0; --p) {
-                const double u = lane < p ? s_u[(b + p) * kBackLd + b + lane] : 0.0;
-                if (lane == p) xi = mid_range(xi) && mid_range(xi * rd) ? div_by(xi, d, rd) : xi / d;
-                const double xp = __shfl_sync(0xffffffffu, xi, p);
-                if (lane < p) xi = fma(-u, xp, xi);
-            }
+            const double x0 = lane < bn ? s_x[b + lane] : 0.0, d = lane < bn ? s_u[(b + lane) * kBackLd + b + lane] : 1.0;
+            const double rd = copysign(rcp_pos(fabs(d)), d);
+            auto solve = [&](auto quotient) {
+                double xi = x0;
+                for (int p = bn - 1; p >= 0; --p) {
+                    const double u = lane < p ? s_u[(b + p) * kBackLd + b + lane] : 0.0;
+                    if (lane == p) xi = quotient(xi);
+                    const double xp = __shfl_sync(0xffffffffu, xi, p);
+                    if (lane < p) xi = fma(-u, xp, xi);
+                }
+                return xi;
+            };
+            bool ok = mid_range(d);
+            double xi = solve([&](double v) {
+                const double q = div_by(v, d, rd);
+                ok = ok && mid_range(v) && mid_range(q);
+                return q;
+            });
+            if (__any_sync(0xffffffffu, !ok && lane < bn)) xi = solve([&](double v) { return v / d; });
             if (lane < bn) s_x[b + lane] = xi;
         }
         __syncthreads();

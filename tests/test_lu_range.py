@@ -20,8 +20,8 @@ def dgesv(A, b):
 
 
 # the largest number, both sides of 2^1022 (where the reciprocal leaves the
-# normal range), of the smallest normal number and of the lines at 1e+-290, subnormals
-ENDS = [1.7976931348623157e308, -1e308, 4.5e307, 4.4e307, 1e300, 1.1e290, 0.9e290, 3.0, -1.0, 1.1e-290, 0.9e-290,
+# normal range), of the smallest normal number and of the lines at 2^960 and 2^-959, subnormals
+ENDS = [1.7976931348623157e308, -1e308, 4.5e307, 4.4e307, 1e300, 9.8e288, 9.7e288, 3.0, -1.0, 1.1e-289, 1.0e-289,
         1e-300, 2.3e-308, -2.2e-308, 1e-308, 1e-310, 5e-324]
 
 
@@ -60,3 +60,16 @@ def test_scaled_system(scale):
     x, _, info = dgesv(A * scale, b * scale)
     assert info == 0
     assert np.linalg.norm(A @ x - b) <= n * 2.0 ** -52 * np.linalg.norm(A) * np.linalg.norm(x)
+
+
+@pytest.mark.parametrize("n", [2, 33, 150])
+def test_subnormal_pivots(n):
+    """Subnormal pivots above other rows (LAPACK's dgetf2 divides there): a lower
+    triangle of ones and a diagonal, both times 2^-1050; every step is exact."""
+    s = 2.0 ** -1050
+    x0 = np.random.default_rng(n).integers(-8, 9, n).astype(np.float64)
+    tri = np.tril(np.ones((n, n)))
+    for A in (tri, np.diag(np.arange(1.0, n + 1))):
+        for rows in (np.arange(n), np.arange(n)[::-1]):  # as they stand, and every pivot a swap
+            x, _, info = dgesv(A[rows] * s, (A @ x0)[rows] * s)
+            assert info == 0 and np.array_equal(x, x0)
