@@ -133,6 +133,8 @@ struct ForwardStep {
     }
 };
 
+constexpr double kFormsMaxC = 1e100;  // largest |R0|^2 at which moments_fp64 uses reciprocals
+
 template <int N>
 __device__ __forceinline__ void moments_fp64(double b, double c, double *I, double *J, double *S) {
     constexpr int K = N + 3;
@@ -157,6 +159,16 @@ __device__ __forceinline__ void moments_fp64(double b, double c, double *I, doub
         S[0] = fadd(fdiv(-4.0, fmul(p2, p2)), fdiv(4.0, fmul(m2, m2)));
         S[1] = fsub(fadd(fdiv(-8.0, fmul(3.0, fmul(p2, p))), fdiv(8.0, fmul(3.0, fmul(m2, m)))),
                     fmul(fmul(b, 0.5), S[0]));
+    } else if (c > kFormsMaxC) {
+        // the products of d, ue and ub overflow from c = 10^122 on, and a quotient
+        // by infinity is zero, which the reciprocals below do not give
+        const double ue3 = fmul(fmul(ue, ue), ue), ub3 = fmul(fmul(ub, ub), ub), d3 = fmul(3.0, d), d6 = fmul(6.0, d);
+        J[0] = fsub(fdiv(te, fmul(d, ue)), fdiv(tb, fmul(d, ub)));
+        J[1] = fsub(j1c, fmul(fmul(b, 0.5), J[0]));
+        S[0] = fadd(fsub(fdiv(fadd(2.0, b), fmul(d6, ue3)), fdiv(fadd(-2.0, b), fmul(d6, ub3))),
+                    fmul(fdiv(2.0, d3), J[0]));
+        S[1] = fsub(fadd(fdiv(-fadd(b, fmul(2.0, c)), fmul(d6, ue3)), fdiv(fadd(-b, fmul(2.0, c)), fmul(d6, ub3))),
+                    fmul(fdiv(b, d3), J[0]));
     } else {
         const double due = fmul(d, ue), dub = fmul(d, ub), d3 = fmul(3.0, d), d6 = fmul(6.0, d);
         const double de = fmul(d6, fmul(fmul(ue, ue), ue)), db = fmul(d6, fmul(fmul(ub, ub), ub));
