@@ -157,10 +157,12 @@ __global__ void __launch_bounds__(kThreads) start_kernel(int64_t n, const T *r, 
         c->g[0] = beta;
         c->k = 0;
         c->hnext = beta;
-        c->stop = !isfinite(beta) || !isfinite(c->bn) ? kStopNaN
-                  : c->bn == 0.0                      ? kStopZeroRhs
-                  : beta == 0.0                       ? kStopTol
-                                                      : 0;
+        // |b| first: without a right-hand side x = 0, whatever the start is
+        c->stop = !isfinite(c->bn)   ? kStopNaN
+                  : c->bn == 0.0     ? kStopZeroRhs
+                  : !isfinite(beta)  ? kStopNaN
+                  : beta == 0.0      ? kStopTol
+                                     : 0;
         if (beta == 0.0) c->bea = 0.0;
         volatile ArnoldiStat *out = stat;
         out->stop = c->stop;

@@ -103,8 +103,8 @@ cudaError_t Gmres<VT>::solve_device(const StopOp &A, const StopOp *P, const VT *
         return launch_arnoldi_start<VT>(n_, r, w_, V_, m, ctrl_, tol, iterMax, kind, cpart_, rb_.counter, rb_.max_blocks,
                                         dstat_ + kArnoldiMax, st_);
     };
-    auto resid = [&](const VT *xv) -> cudaError_t {  // w_ = b - A xv
-        RF_TRY(A(xv, w_, nullptr));
+    auto resid = [&](const VT *xv, const int *stop_at) -> cudaError_t {  // w_ = b - A xv
+        RF_TRY(A(xv, w_, stop_at));
         res->matvecs++;
         res->launches++;
         return launch_bmr<VT>(n_, b, w_, st_);
@@ -114,7 +114,7 @@ cudaError_t Gmres<VT>::solve_device(const StopOp &A, const StopOp *P, const VT *
     if (x_is_zero) {
         RF_TRY(cudaMemsetAsync(x, 0, sizeof(VT) * n_, st_));
     } else {
-        RF_TRY(resid(x));
+        RF_TRY(resid(x, stop));  // with |b| = 0 the product returns at once, and no step follows
         RF_TRY(start(w_, kStartFrom));
     }
     int last_stop = 0;
@@ -162,8 +162,10 @@ cudaError_t Gmres<VT>::solve_device(const StopOp &A, const StopOp *P, const VT *
                 if (!read_start()) done = m - 1;
             }
             if (start_stop > 0) {
-                // every step of this cycle returned at once
-                for (int q = 0; q < queued; ++q) {
+                // every step of this cycle returned at once, and without a
+                // right-hand side the first residual's product too
+                const int skipped = queued + (start_stop == kStopZeroRhs && !x_is_zero ? 1 : 0);
+                for (int q = 0; q < skipped; ++q) {
                     res->matvecs--;
                     if (on_skipped_product) on_skipped_product();
                 }
@@ -200,7 +202,7 @@ cudaError_t Gmres<VT>::solve_device(const StopOp &A, const StopOp *P, const VT *
                 return cudaSuccess;
             }
             // the estimate met the tolerance (or the budget is spent): the true residual decides
-            RF_TRY(resid(xcur_));
+            RF_TRY(resid(xcur_, nullptr));
             double tn, bn;
             RF_TRY(launch_dot<VT>(n_, w_, w_, hcol_, rb_, st_));
             res->launches++;
@@ -224,7 +226,7 @@ cudaError_t Gmres<VT>::solve_device(const StopOp &A, const StopOp *P, const VT *
         // restart from the residual of the updated x, without a product where
         // the cycle's basis may give it (arnoldi.cu)
         if (check_failed) {
-            RF_TRY(resid(x));
+            RF_TRY(resid(x, nullptr));
             RF_TRY(start(w_, kStartFrom));
         } else {
             RF_TRY(start(w_, kStartBasis));

@@ -248,7 +248,14 @@ struct Solver {
             s.x[r] = a.x[r0 + r];
             s.b[r] = a.b[r0 + r];
         }
-        __syncthreads();
+        // without a right-hand side (one fiber, or no external force) x = 0; every
+        // CTA looks at all of b, as no barrier costs less
+        bool any = false;
+        for (int r = threadIdx.x; r < (int)a.n; r += kThreads) any = any || a.b[r] != 0.0;
+        if (!__syncthreads_or(any)) {
+            for (int r = threadIdx.x; r < rows; r += kThreads) a.x[r0 + r] = 0.0;
+            return leave(kSmallOk);
+        }
         product(a.x, 1.0, true);
         ++st.matvecs;
         publish(a.w, s.w);
