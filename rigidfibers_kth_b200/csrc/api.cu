@@ -428,7 +428,7 @@ rf_status rf_create(const rf_params *p, const double *positions, const double *o
     }
     h->asm_chunk = (M + chunks - 1) / chunks;
     h->asm_chunks = (M + h->asm_chunk - 1) / h->asm_chunk;
-    h->vel_chunks = rf::pair_sum_chunks(M, h->sm_count);
+    h->vel_chunks = rf::pair_sum_chunks(M, h->LQ, h->sm_count);
     h->vel_chunk = (M + h->vel_chunks - 1) / h->vel_chunks;
     h->asm64 = prec == RF_PREC_FP64 && p->use_analytical_integration != 0 && rf::assemble64_supported(N);
     if (h->asm64) {

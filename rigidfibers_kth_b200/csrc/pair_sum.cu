@@ -11,8 +11,8 @@
 //     . IF); k >= 2: gamma_k (IF - E_k t (t . IF))).  Reference: mat_prod,
 //     fortran/matrix_assembly.f90:159-265.  A is never formed: memory O(M).
 //
-// Mapping.  A CTA owns four targets and a chunk of sources, thread (ti, q) one
-// target point; the sources are staged in shared memory in batches, with what
+// Mapping.  A CTA owns some targets (four of the usual 24 points) and a chunk of
+// sources, thread (ti, q) one target point; the sources are staged in shared memory in batches, with what
 // all points of the GPU share of a source formed once per CTA: the force's
 // monomial coefficients F_p (P_l written out) and pb . F_p, or for the numeric
 // integral its weighted values at the source's Gauss points.  Then, with u_p
@@ -38,14 +38,25 @@ namespace rf {
 
 namespace {
 
-constexpr int kTI = 4;      // targets per CTA
+// Targets per CTA: at least four, and at fewer than 24 points a fiber as many as
+// fill two or three warps, whichever leaves fewer lanes without a point (four
+// targets left 20 of 32 at 3 points, 28 of 64 at 9, 16 of 64 at 12).
+// Velocities, M = 800, N = 5: 3 points 357 -> 156 us, 9 points 651 -> 370, 12
+// points 630 -> 481, 18 points 805 -> 742.
+constexpr int kPoints = 96;
+constexpr int kMinTI = 4;
+constexpr int targets_of(int LQ) {
+    const int two = 64 / LQ, three = kPoints / LQ;
+    return three <= kMinTI ? kMinTI : two >= kMinTI && 3 * two >= 2 * three ? two : three;
+}
+static_assert(targets_of(3) == 32 && targets_of(9) == 7 && targets_of(15) == 4 && targets_of(24) == 4, "");
 constexpr int kBatch = 16;  // analytic: sources staged at a time
 constexpr int kBatchNum = 4;
 
 constexpr int round32(int v) { return (v + 31) / 32 * 32; }
 
 struct PairSumArgs {
-    int M, LQ;
+    int M, LQ, TI;             // TI: targets per CTA
     int t0, t1;                // target fibers [t0, t1)
     const double *pos, *ori;
     const double *coeffs;      // n: the sources' coefficients
@@ -95,7 +106,7 @@ __global__ void __launch_bounds__(MAXT, MINB) pair_sum_kernel(PairSumArgs a) {
     constexpr int NL = N + 1;
     using Src = SourceA<N>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int LQ = a.LQ, nthreads = blockDim.x, tid = threadIdx.x;
+    const int LQ = a.LQ, TI = a.TI, nthreads = blockDim.x, tid = threadIdx.x;
     const Tables &tab = *a.tab;
     // analytic: kBatch sources, then the recursion's table; numeric: kBatchNum
     // x LQ x (point, weighted force); at the end: TI x LQ x 3 sums
@@ -105,10 +116,10 @@ __global__ void __launch_bounds__(MAXT, MINB) pair_sum_kernel(PairSumArgs a) {
     double *s_u = reinterpret_cast<double *>(smem_raw);
     if (!NUMERIC)
         for (int t = tid; t < Far<N>::kCoef; t += nthreads) s_far[t] = Far<N>::coef(t);
-    const int i0 = a.t0 + blockIdx.x * kTI;  // first target of the tile (global index)
+    const int i0 = a.t0 + blockIdx.x * TI;  // first target of the tile (global index)
     const int ti = tid / LQ, q = tid - ti * LQ;
     const int i = i0 + ti;
-    const bool live = ti < kTI && i < a.t1;
+    const bool live = ti < TI && i < a.t1;
     double xb[3] = {0.0, 0.0, 0.0};
     if (live) {
         const double *xc = a.pos + 3 * i, *tc = a.ori + 3 * i;
@@ -198,14 +209,14 @@ __global__ void __launch_bounds__(MAXT, MINB) pair_sum_kernel(PairSumArgs a) {
         }
     }
     __syncthreads();
-    if (ti < kTI) {
+    if (ti < TI) {
 #pragma unroll
         for (int c = 0; c < 3; ++c) s_u[3 * tid + c] = us[c];
     }
     __syncthreads();
     if (!MATFREE) {
         // IF_k = sum_q w_q P_k(s_q) u_q, k = 0, 1
-        for (int t = tid; t < kTI * 6; t += nthreads) {
+        for (int t = tid; t < TI * 6; t += nthreads) {
             const int gt = t / 6, k = t % 6 / 3, c = t % 3;
             if (i0 + gt >= a.t1) continue;
             double s = 0.0;
@@ -217,7 +228,7 @@ __global__ void __launch_bounds__(MAXT, MINB) pair_sum_kernel(PairSumArgs a) {
         }
         return;
     }
-    for (int t = tid; t < kTI * N; t += nthreads) {
+    for (int t = tid; t < TI * N; t += nthreads) {
         const int gt = t / N, k = t % N + 1;
         const int it = i0 + gt;
         if (it >= a.t1) continue;
@@ -251,13 +262,13 @@ constexpr int kMinB = 5;
 
 template <int N, bool NUMERIC, bool MATFREE>
 cudaError_t launch_n(const PairSumArgs &a, int nchunks, cudaStream_t st) {
-    const int threads = round32(kTI * a.LQ);
+    const int threads = round32(a.TI * a.LQ);
     const size_t src = NUMERIC ? sizeof(double) * 6 * kBatchNum * a.LQ
                                : sizeof(SourceA<N>) * kBatch + sizeof(double) * Far<N>::kCoef;
-    const size_t smem = std::max(src, sizeof(double) * 3 * kTI * (size_t)a.LQ);
-    auto kern = threads <= 96 ? pair_sum_kernel<N, NUMERIC, MATFREE, 96, kMinB>
-                              : pair_sum_kernel<N, NUMERIC, MATFREE, kTI * kMaxLQ, 2>;
-    kern<<<dim3((a.t1 - a.t0 + kTI - 1) / kTI, nchunks), threads, smem, st>>>(a);
+    const size_t smem = std::max(src, sizeof(double) * 3 * a.TI * (size_t)a.LQ);
+    auto kern = threads <= kPoints ? pair_sum_kernel<N, NUMERIC, MATFREE, kPoints, kMinB>
+                                   : pair_sum_kernel<N, NUMERIC, MATFREE, kMinTI * kMaxLQ, 2>;
+    kern<<<dim3((a.t1 - a.t0 + a.TI - 1) / a.TI, nchunks), threads, smem, st>>>(a);
     return cudaGetLastError();
 }
 
@@ -274,18 +285,19 @@ cudaError_t launch_pair_sum(const PairSumArgs &a, int N, bool numeric, int nchun
 
 }  // namespace
 
-int pair_sum_chunks(int M, int sm_count) {
-    return pick_chunks(M, (M + kTI - 1) / kTI, kMinB * (int64_t)sm_count, 1);
+int pair_sum_chunks(int M, int LQ, int sm_count) {
+    const int TI = targets_of(LQ);
+    return pick_chunks(M, (M + TI - 1) / TI, kMinB * (int64_t)sm_count, 1);
 }
 
 cudaError_t launch_velocity(const VelArgs &a, bool numeric, int nchunks, cudaStream_t st) {
-    return launch_pair_sum<false>({a.M, a.LQ, a.t0, a.t1, a.pos, a.ori, a.coeffs, a.tab, a.part, 6LL * a.M, a.chunk},
+    return launch_pair_sum<false>({a.M, a.LQ, targets_of(a.LQ), a.t0, a.t1, a.pos, a.ori, a.coeffs, a.tab, a.part, 6LL * a.M, a.chunk},
                                   a.N, numeric, nchunks, st);
 }
 
 cudaError_t launch_matfree(const MatfreeArgs &a, bool numeric, int nchunks, const double *x, double *y,
                            cudaStream_t st) {
-    cudaError_t e = launch_pair_sum<true>({a.M, a.LQ, 0, a.M, a.pos, a.ori, a.x, a.tab, a.part, a.n, a.chunk}, a.N,
+    cudaError_t e = launch_pair_sum<true>({a.M, a.LQ, targets_of(a.LQ), 0, a.M, a.pos, a.ori, a.x, a.tab, a.part, a.n, a.chunk}, a.N,
                                           numeric, nchunks, st);
     if (e != cudaSuccess) return e;
     matfree_finish_kernel<<<(unsigned)((a.n + 255) / 256), 256, 0, st>>>(a.n, nchunks, a.part, x, y);

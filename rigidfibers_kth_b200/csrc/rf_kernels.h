@@ -169,7 +169,7 @@ struct VelArgs {
     int chunk;
 };
 cudaError_t launch_velocity(const VelArgs &a, bool numeric, int nchunks, cudaStream_t st);
-int pair_sum_chunks(int M, int sm_count);  // source chunks of launch_velocity and launch_matfree
+int pair_sum_chunks(int M, int LQ, int sm_count);  // source chunks of launch_velocity and launch_matfree
 
 // Matrix-free FP64 product y = A x (pair_sum.cu), the reference's mat_prod.
 struct MatfreeArgs {
