@@ -223,10 +223,16 @@ __device__ __forceinline__ void moments_fp64(double b, double c, double *I, doub
 // like c, 4e-9 at c = 10^6) would show against the recursion likewise.
 // The start (far_top): zero starting values reach n <= 7 damped by c^(-n/2)
 // times a polynomial in n, and an even start is closer than an odd one, so it
-// falls with c.  Relative to J_0, 40-digit evaluation, n <= 7, at the lower
-// end of every range: J_n within 7e-13 for |b| up to 0.9 of its largest value
-// and 4e-12 at the edge of the cone; the start at 27 leaves 3e-11 at |b| = 0.9
-// of its largest value at c = 10.
+// falls with c.  The lines lie where the Legendre combinations (m <= 5) of I_n,
+// J_n, S_n, relative to I_0, J_0, S_0 and against 40 digits, have a mean, median
+// and largest error over isotropic directions that are no larger than those of
+// the reference's formulas in FP64 (its start at 27, the closed forms'
+// cancellation): mean of J just above the lines 16, 45, 65, 105, 190, 420 9.6e-13,
+// 7e-16, 1e-15, 2e-15, 5e-15, 9e-15 (reference 2.2e-12, 8e-15, 2e-14, 2e-14,
+// 6e-14, 1e-13), and at 10 and 13 1.2e-12 and 6e-13 (2e-10, 1e-11).  N = 8 with
+// its four steps more likewise.  Lines at 16, 20, 30, 48, 80, 150 left up to 100
+// times the reference's error; the higher starts cost 0.5 ms of an assembly and
+// 0.6 ms of the velocities at M = 4000 (21.8 and 14.4 ms).
 constexpr double kFarC = 10.0;
 constexpr double kFarMaxC = 4096.0;
 constexpr double kAxisRatio = 1e-3, kAxisRatioNear = 1e-2;
@@ -234,7 +240,7 @@ __device__ __forceinline__ bool far_point(double b, double c) {
     return c >= kFarC && c < kFarMaxC && fma(-0.25 * b, b, c) >= (c < 16.0 ? kAxisRatioNear : kAxisRatio) * c;
 }
 __device__ __forceinline__ int far_top(float c) {
-    return 16 + 2 * ((c < 150.f) + (c < 80.f) + (c < 48.f) + (c < 30.f) + (c < 20.f) + (c < 16.f) + (c < 13.f));
+    return 16 + 2 * ((c < 420.f) + (c < 190.f) + (c < 105.f) + (c < 65.f) + (c < 45.f) + (c < 16.f) + (c < 13.f));
 }
 
 // Step n: I_n = -(1 + r/2) (b/c) I_{n+1} - (1 + r) (1/c) I_{n+2} + r w, r =
