@@ -194,6 +194,9 @@ __global__ void __launch_bounds__(MAXT, MINB) pair_sum_kernel(PairSumArgs a) {
             } else {
                 const double *y = s_num + 6 * LQ * r;
                 const double e2 = 2.0 * eps2, e6 = 6.0 * eps2;
+                // the source's own sum first: 48 additions a source straight into the
+                // running sum left rms errors 1.5 times as large (M = 2000)
+                double u0 = 0.0, u1 = 0.0, u2 = 0.0;
 #pragma unroll 2
                 for (int k = 0; k < LQ; ++k, y += 6) {
                     const double Rx = xb[0] - y[0], Ry = xb[1] - y[1], Rz = xb[2] - y[2];
@@ -201,10 +204,13 @@ __global__ void __launch_bounds__(MAXT, MINB) pair_sum_kernel(PairSumArgs a) {
                     const double ir2 = ir * ir, ir3 = ir2 * ir;
                     const double diag = fma(e2, ir3, ir), off = ir3 * fma(-e6, ir2, 1.0);
                     const double rf = fma(Rx, y[3], fma(Ry, y[4], Rz * y[5])) * off;
-                    us[0] = fma(diag, y[3], fma(Rx, rf, us[0]));
-                    us[1] = fma(diag, y[4], fma(Ry, rf, us[1]));
-                    us[2] = fma(diag, y[5], fma(Rz, rf, us[2]));
+                    u0 = fma(diag, y[3], fma(Rx, rf, u0));
+                    u1 = fma(diag, y[4], fma(Ry, rf, u1));
+                    u2 = fma(diag, y[5], fma(Rz, rf, u2));
                 }
+                us[0] += u0;
+                us[1] += u1;
+                us[2] += u2;
             }
         }
     }
