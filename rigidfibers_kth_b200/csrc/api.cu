@@ -26,12 +26,12 @@ cudaError_t dalloc(T **p, size_t count) {
 // y = A x (r null) or y = r - A x over the FP32 matrix of the FP32 and mixed
 // paths: its own FP32 storage, or the two 16-bit planes of the mixed BF16 path
 template <typename X, typename ACC, typename Y>
-cudaError_t fp32_gemv(rf_handle *h, const X *x, Y *y, const Y *r, ACC *work, const int *stop = nullptr) {
+cudaError_t fp32_gemv(rf_handle *h, const X *x, Y *y, const Y *r, rf::GemvWork<ACC> work, const int *stop = nullptr) {
     if (h->A16lo)
         return rf::launch_gemv<rf::SplitF32, X, ACC, Y>(reinterpret_cast<const rf::SplitF32 *>(h->A16), h->lda, h->n,
-                                                        h->n, x, y, r, work, h->work_elems, h->sm_count, h->stream,
+                                                        h->n, x, y, r, work, h->sm_count, h->stream,
                                                         stop, h->a_plane);
-    return rf::launch_gemv<float, X, ACC, Y>(h->A32, h->lda, h->n, h->n, x, y, r, work, h->work_elems, h->sm_count,
+    return rf::launch_gemv<float, X, ACC, Y>(h->A32, h->lda, h->n, h->n, x, y, r, work, h->sm_count,
                                              h->stream, stop);
 }
 
@@ -46,7 +46,7 @@ void free_all(rf_handle *h) {
         cudaFree(h->W[i]);
     }
     void *ptrs[] = {h->tab, h->A64, h->LU, h->lu_r, h->lu_piv, h->lu_info, h->mfpart, h->mvx, h->A32, h->A16, h->b, h->x, h->PV64, h->PW64,
-                    h->PV32, h->PW32, h->vpart, h->pvx, h->pwx, h->work64, h->work32, h->r64, h->r32,
+                    h->PV32, h->PW32, h->vpart, h->pvx, h->pwx, h->work64, h->work32.p, h->r64, h->r32,
                     h->d32, h->x32, h->Pblocks, h->knn, h->mlp_w, h->mlp_wtc, h->mlp_err, h->feat, h->mlp_h1, h->mlp_h2, h->mlp_out,
                     h->dscal, h->rb.partials, h->rb.counter, h->near_bits, h->near_list, h->near_cnt,
                     h->far_contr, h->near_contr, h->near_pref, h->near_off, h->near_total, h->nearbuf};
@@ -490,7 +490,10 @@ rf_status rf_create(const rf_params *p, const double *positions, const double *o
                               h->small ? rf::gmres_small_work(h->n, h->sm_count) : 0});
     CKC(dalloc(&h->work64, h->work_elems), "alloc workspace");
     h->bpart = h->velpart = h->work64;
-    if (prec != RF_PREC_FP64) CKC(dalloc(&h->work32, gemv_elems), "alloc matvec workspace");
+    if (prec != RF_PREC_FP64) {
+        h->work32.elems = gemv_elems;
+        CKC(dalloc(&h->work32.p, gemv_elems), "alloc matvec workspace");
+    }
     CKC(dalloc(&h->dscal, 8), "alloc scalars");
     CKC(cudaMallocHost(&h->hscal, 8 * sizeof(double)), "alloc pinned scalars");
     h->rb.max_blocks = 1024;
@@ -776,7 +779,7 @@ rf_status rf_solve_system(rf_handle *h) {
         CK(h, cudaMemcpyAsync(h->x, y, sizeof(double) * h->n, cudaMemcpyDeviceToDevice, st), "direct solver");
         // backward error |b - A x| / |b| for the statistics
         CK(h, (rf::launch_gemv<double, double, double, double>(h->A64, h->lda, h->n, h->n, h->x, h->lu_r, h->b,
-                                                                h->work64, h->work_elems, h->sm_count, st)),
+                                                                h->gemv64(), h->sm_count, st)),
            "direct solver residual");
         CK(h, rf::launch_dot<double>(h->n, h->lu_r, h->lu_r, h->dscal, h->rb, st), "direct solver residual");
         CK(h, rf::launch_dot<double>(h->n, h->b, h->b, h->dscal + 1, h->rb, st), "direct solver residual");
@@ -806,14 +809,14 @@ rf_status rf_solve_system(rf_handle *h) {
                 // this shard's rows, then the row blocks of every shard
                 cudaError_t e = timed_product(h, 8.0 * h->lda * h->n, [&] {
                     return rf::launch_gemv<double, double, double, double>(h->A64, h->lda, h->n_loc, h->n, in,
-                                                                            h->shard_send, nullptr, h->work64,
-                                                                            h->work_elems, h->sm_count, h->stream, stop);
+                                                                            h->shard_send, nullptr, h->gemv64(),
+                                                                            h->sm_count, h->stream, stop);
                 });
                 return e == cudaSuccess ? rf::shard_allgather(h, out, 3 * h->N, h->shard_send) : e;
             }
             return timed_product(h, 8.0 * h->lda * h->n, [&] {
                 return rf::launch_gemv<double, double, double, double>(h->A64, h->lda, h->n, h->n, in, out, nullptr,
-                                                                       h->work64, h->work_elems, h->sm_count,
+                                                                       h->gemv64(), h->sm_count,
                                                                        h->stream, stop);
             });
         };
@@ -948,7 +951,7 @@ rf_status rf_solve_system(rf_handle *h) {
             return timed_product(h, (bf16 ? 2.0 : 4.0) * h->lda * h->n, [&] {
                 if (bf16)
                     return rf::launch_gemv<__nv_bfloat16, float, float, float>(h->A16, h->lda, h->n, h->n, in, out,
-                                                                               nullptr, h->work32, h->work_elems,
+                                                                               nullptr, h->work32,
                                                                                h->sm_count, h->stream);
                 return fp32_gemv<float, float, float>(h, in, out, nullptr, h->work32);
             });
@@ -964,7 +967,7 @@ rf_status rf_solve_system(rf_handle *h) {
             return timed_product(h, (bf16 ? 2.0 : 4.0) * h->lda * h->n, [&] {
                 if (bf16)
                     return rf::launch_gemv<__nv_bfloat16, float, float, float>(h->A16, h->lda, h->n, h->n, in, out,
-                                                                               nullptr, h->work32, h->work_elems,
+                                                                               nullptr, h->work32,
                                                                                h->sm_count, h->stream, stop);
                 return fp32_gemv<float, float, float>(h, in, out, nullptr, h->work32, stop);
             });
@@ -988,7 +991,7 @@ rf_status rf_solve_system(rf_handle *h) {
         auto residual = [&]() -> cudaError_t {  // r64 = b - A32 x (FP64 accumulation)
             h->launches += 2;
             h->stats.matvecs++;
-            return fp32_gemv<double, double, double>(h, h->x, h->r64, h->b, h->work64);
+            return fp32_gemv<double, double, double>(h, h->x, h->r64, h->b, h->gemv64());
         };
         double bn = 0.0, rn = 0.0;
         cudaError_t e = norm_of(h->b, &bn);
@@ -1113,17 +1116,17 @@ rf_status rf_update_velocities(rf_handle *h) {
         const int64_t m3 = 3LL * h->M;
         if (h->PV64) {
             CK(h, (rf::launch_gemv<double, double, double, double>(h->PV64, h->ldp, m3, h->n, h->x, h->pvx, nullptr,
-                                                                    h->work64, h->work_elems, h->sm_count, st)),
+                                                                    h->gemv64(), h->sm_count, st)),
                "velocity panel");
             CK(h, (rf::launch_gemv<double, double, double, double>(h->PW64, h->ldp, m3, h->n, h->x, h->pwx, nullptr,
-                                                                    h->work64, h->work_elems, h->sm_count, st)),
+                                                                    h->gemv64(), h->sm_count, st)),
                "velocity panel");
         } else {
             CK(h, (rf::launch_gemv<float, double, double, double>(h->PV32, h->ldp, m3, h->n, h->x, h->pvx, nullptr,
-                                                                   h->work64, h->work_elems, h->sm_count, st)),
+                                                                   h->gemv64(), h->sm_count, st)),
                "velocity panel");
             CK(h, (rf::launch_gemv<float, double, double, double>(h->PW32, h->ldp, m3, h->n, h->x, h->pwx, nullptr,
-                                                                   h->work64, h->work_elems, h->sm_count, st)),
+                                                                   h->gemv64(), h->sm_count, st)),
                "velocity panel");
         }
         CK(h, rf::launch_velocity_reuse_finish(h->M, h->T[h->cur], h->tab, h->pvx, h->pwx, h->vpart, h->vpart_chunks,
@@ -1293,15 +1296,15 @@ rf_status rf_matvec(rf_handle *h, const double *x, double *y) {
     cudaError_t e = cudaMemcpyAsync(dx, x, h->n * 8, cudaMemcpyHostToDevice, h->stream);
     if (e == cudaSuccess) {
         if (h->A64)
-            e = rf::launch_gemv<double, double, double, double>(h->A64, h->lda, h->n, h->n, dx, dy, nullptr, h->work64,
-                                                                h->work_elems, h->sm_count, h->stream);
+            e = rf::launch_gemv<double, double, double, double>(h->A64, h->lda, h->n, h->n, dx, dy, nullptr,
+                                                                h->gemv64(), h->sm_count, h->stream);
         else if (h->A16)
             e = rf::launch_gemv<__nv_bfloat16, double, double, double>(h->A16, h->lda, h->n, h->n, dx, dy, nullptr,
-                                                                       h->work64, h->work_elems, h->sm_count,
+                                                                       h->gemv64(), h->sm_count,
                                                                        h->stream);
         else
-            e = rf::launch_gemv<float, double, double, double>(h->A32, h->lda, h->n, h->n, dx, dy, nullptr, h->work64,
-                                                               h->work_elems, h->sm_count, h->stream);
+            e = rf::launch_gemv<float, double, double, double>(h->A32, h->lda, h->n, h->n, dx, dy, nullptr,
+                                                               h->gemv64(), h->sm_count, h->stream);
         h->launches += 2;
     }
     if (e == cudaSuccess) e = cudaMemcpyAsync(y, dy, h->n * 8, cudaMemcpyDeviceToHost, h->stream);
@@ -1478,17 +1481,17 @@ rf_status rf_profile_matvec(rf_handle *h, int32_t reps, double *ms_per_product, 
     for (int r = 0; r < reps && e == cudaSuccess; ++r) {
         if (h->A64) {
             e = rf::launch_gemv<double, double, double, double>(h->A64, h->lda, n, n, (double *)xv, (double *)yv,
-                                                                nullptr, h->work64, h->work_elems, h->sm_count,
+                                                                nullptr, h->gemv64(), h->sm_count,
                                                                 h->stream);
             elem = 8.0;
         } else if (h->A16) {
             e = rf::launch_gemv<__nv_bfloat16, float, float, float>(h->A16, h->lda, n, n, (float *)xv, (float *)yv,
-                                                                    nullptr, h->work32, h->work_elems, h->sm_count,
+                                                                    nullptr, h->work32, h->sm_count,
                                                                     h->stream);
             elem = 2.0;
         } else {
             e = rf::launch_gemv<float, float, float, float>(h->A32, h->lda, n, n, (float *)xv, (float *)yv, nullptr,
-                                                            h->work32, h->work_elems, h->sm_count, h->stream);
+                                                            h->work32, h->sm_count, h->stream);
             elem = 4.0;
         }
         h->launches += 2;

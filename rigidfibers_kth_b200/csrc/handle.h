@@ -72,8 +72,9 @@ struct rf_handle {
     double *pvx = nullptr, *pwx = nullptr;
     // matvec workspace
     double *work64 = nullptr;  // FP64 partial sums that live within one call
-    float *work32 = nullptr;
-    int64_t work_elems = 0;
+    int64_t work_elems = 0;    // doubles in it
+    rf::GemvWork<double> gemv64() const { return {work64, work_elems}; }
+    rf::GemvWork<float> work32;  // products with FP32 sums (not made for the FP64 method)
     bool small = false;        // small FP64 system: GMRES in one kernel (gmres_small.cu), in work64 and dscal[2..5]
     // solver
     std::unique_ptr<rf::Gmres<double>> gm64;

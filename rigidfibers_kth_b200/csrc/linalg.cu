@@ -247,49 +247,36 @@ int64_t gemv_work_elems(int64_t m, int sm_count, int elem_bytes) {
 }
 
 template <typename S, typename X, typename ACC, typename Y>
-cudaError_t launch_gemv(const S *A, int64_t lda, int64_t m, int64_t k, const X *x, Y *y, const Y *r, ACC *work,
-                        int64_t work_elems, int sm_count, cudaStream_t st, const int *stop, int64_t plane) {
+cudaError_t launch_gemv(const S *A, int64_t lda, int64_t m, int64_t k, const X *x, Y *y, const Y *r,
+                        GemvWork<ACC> work, int sm_count, cudaStream_t st, const int *stop, int64_t plane) {
     constexpr int VEC = Vec16<S>::kVec;
     const int64_t tiles = (lda + (int64_t)kGemvThreads * VEC - 1) / ((int64_t)kGemvThreads * VEC);
     const int64_t mpad = tiles * kGemvThreads * VEC;
     int splits = gemv_splits(m, k, VEC, gemv_slots<S, X, ACC>(sm_count));
-    while (splits > 1 && (int64_t)splits * mpad > work_elems) --splits;
-    if ((int64_t)splits * mpad > work_elems) return cudaErrorInvalidValue;
+    while (splits > 1 && (int64_t)splits * mpad > work.elems) --splits;
+    if ((int64_t)splits * mpad > work.elems) return cudaErrorInvalidValue;
     const int64_t cps = (k + splits - 1) / splits;
     dim3 grid((unsigned)tiles, (unsigned)splits);
     cudaError_t e = launch_pdl(gemv_partial_kernel<S, X, ACC>, grid, dim3(kGemvThreads), 0, st, A, lda, m, k, x, cps,
-                               work, mpad, stop, plane);
+                               work.p, mpad, stop, plane);
     if (e != cudaSuccess) return e;
     constexpr int ROWS = 32 * 16 / (int)sizeof(ACC);
     static_assert(kGemvThreads * VEC % ROWS == 0, "whole groups of rows in mpad");
     return launch_pdl(gemv_reduce_kernel<ACC, Y>, dim3((unsigned)((m + ROWS - 1) / ROWS)), dim3(32 * kRedSlices), 0, st,
-                      static_cast<const ACC *>(work), splits, mpad, m, y, r, stop);
+                      static_cast<const ACC *>(work.p), splits, mpad, m, y, r, stop);
 }
 
-template cudaError_t launch_gemv<double, double, double, double>(const double *, int64_t, int64_t, int64_t,
-                                                                 const double *, double *, const double *,
-                                                                 double *, int64_t, int, cudaStream_t, const int *, int64_t);
-template cudaError_t launch_gemv<float, double, double, double>(const float *, int64_t, int64_t, int64_t,
-                                                                const double *, double *, const double *,
-                                                                double *, int64_t, int, cudaStream_t, const int *, int64_t);
-template cudaError_t launch_gemv<float, float, float, float>(const float *, int64_t, int64_t, int64_t,
-                                                             const float *, float *, const float *, float *,
-                                                             int64_t, int, cudaStream_t, const int *, int64_t);
-template cudaError_t launch_gemv<__nv_bfloat16, float, float, float>(const __nv_bfloat16 *, int64_t, int64_t,
-                                                                     int64_t, const float *, float *,
-                                                                     const float *, float *, int64_t, int,
-                                                                     cudaStream_t, const int *, int64_t);
-template cudaError_t launch_gemv<__nv_bfloat16, double, double, double>(const __nv_bfloat16 *, int64_t, int64_t,
-                                                                        int64_t, const double *, double *,
-                                                                        const double *, double *, int64_t, int,
-                                                                        cudaStream_t, const int *, int64_t);
-template cudaError_t launch_gemv<SplitF32, double, double, double>(const SplitF32 *, int64_t, int64_t, int64_t,
-                                                                   const double *, double *, const double *,
-                                                                   double *, int64_t, int, cudaStream_t, const int *,
-                                                                   int64_t);
-template cudaError_t launch_gemv<SplitF32, float, float, float>(const SplitF32 *, int64_t, int64_t, int64_t,
-                                                                const float *, float *, const float *, float *,
-                                                                int64_t, int, cudaStream_t, const int *, int64_t);
+#define RF_GEMV(S, T)                                                                                                  \
+    template cudaError_t launch_gemv<S, T, T, T>(const S *, int64_t, int64_t, int64_t, const T *, T *, const T *,     \
+                                                 GemvWork<T>, int, cudaStream_t, const int *, int64_t);
+RF_GEMV(double, double)
+RF_GEMV(float, double)
+RF_GEMV(float, float)
+RF_GEMV(__nv_bfloat16, float)
+RF_GEMV(__nv_bfloat16, double)
+RF_GEMV(SplitF32, double)
+RF_GEMV(SplitF32, float)
+#undef RF_GEMV
 
 // ---------------------------------------------------------------------------
 // reductions

@@ -89,7 +89,7 @@ extern "C" rf_status rf_matvec_noalloc(const double *A, int64_t lda, int64_t n, 
     }
     // every partial sum that the reduction reads is written earlier in the
     // same call, so nothing in the array needs to start at zero
-    e = rf::launch_gemv<double, double, double, double>(A, lda, n, n, x, y, nullptr, scratch, kScratchDoubles, sms,
+    e = rf::launch_gemv<double, double, double, double>(A, lda, n, n, x, y, nullptr, {scratch, kScratchDoubles}, sms,
                                                        static_cast<cudaStream_t>(stream));
     if (e != cudaSuccess) {
         cudaGetLastError();

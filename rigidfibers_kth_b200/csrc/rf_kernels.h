@@ -204,9 +204,16 @@ cudaError_t launch_normalize(int M, double *T, cudaStream_t st);
 // stop (optional, device): when *stop != 0 at launch time every CTA returns at
 // once (a product queued ahead for a solve that has finished meanwhile).
 // S = SplitF32: A is the high plane, the low plane `plane` entries further.
+// work: the splits' partial sums; fewer splits where it holds fewer, an error
+// where it does not hold one.
+template <typename ACC>
+struct GemvWork {
+    ACC *p = nullptr;
+    int64_t elems = 0;
+};
 template <typename S, typename X, typename ACC, typename Y>
 cudaError_t launch_gemv(const S *A, int64_t lda, int64_t m, int64_t k, const X *x, Y *y, const Y *r,
-                        ACC *work, int64_t work_elems, int sm_count, cudaStream_t st, const int *stop = nullptr,
+                        GemvWork<ACC> work, int sm_count, cudaStream_t st, const int *stop = nullptr,
                         int64_t plane = 0);
 int64_t gemv_work_elems(int64_t m, int sm_count, int elem_bytes);
 
