@@ -843,10 +843,12 @@ rf_status rf_solve_system(rf_handle *h) {
             const cudaError_t e = rf::launch_gmres_small(sa, h->work64, h->sm_count, st);
             if (e != cudaErrorCooperativeLaunchTooLarge) {
                 CK(h, e, "GMRES");
-                rf::SmallGmresStat *hs = reinterpret_cast<rf::SmallGmresStat *>(h->hscal);
-                CK(h, cudaMemcpyAsync(hs, sa.stat, sizeof(*hs), cudaMemcpyDeviceToHost, st), "GMRES");
+                // the barrier's words and the outcome: dscal[2] and the three after it
+                const unsigned *hb = reinterpret_cast<const unsigned *>(h->hscal);
+                const auto *hs = reinterpret_cast<const rf::SmallGmresStat *>(h->hscal + 1);
+                CK(h, cudaMemcpyAsync(h->hscal, sa.barrier, 8 + sizeof(*hs), cudaMemcpyDeviceToHost, st), "GMRES");
                 CK(h, cudaStreamSynchronize(st), "GMRES");
-                if (hs->info == rf::kSmallTimeout)
+                if (hb[1] || hs->info == rf::kSmallTimeout)
                     return rf::fail(h, RF_ERR_DEVICE_TIMEOUT, "GMRES: a grid barrier timed out");
                 res.info = hs->info == rf::kSmallNaN ? rf::kInfoNaN : hs->info == rf::kSmallBudget ? rf::kInfoBudget : 0;
                 res.iterations = hs->iterations;

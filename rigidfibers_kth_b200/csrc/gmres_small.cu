@@ -3,10 +3,10 @@
 //
 // The flow is the one of gmres.h (fortran/dGMRES.f:491-1495): warm start, CGS2
 // orthogonalisation as in arnoldi.cu, Givens rotations, the true residual when
-// the estimate meets the tolerance and at each restart.  What bounds a small
-// system is the chain of launches: a step of the device-controlled solver is
-// six kernels, 36 us at n = 1500 where the product reads its 18 MB from L2 in
-// about 3.  Here a step's phases are separated by two grid barriers:
+// the estimate meets the tolerance; a restart takes its residual from the
+// cycle's basis, as there.  What bounds a small system is the chain of
+// launches: a step of the device-controlled solver is six kernels, 31 us at n =
+// 1500 where the product reads its 18 MB from L2 in about 3.  Here a step's phases are separated by two grid barriers:
 //   product    a CTA's own rows (up to kSmallRows) of A v, kept in its shared
 //              memory with its rows of the basis, of the basis' products and
 //              of x; partial dot products h1 = V^T w;
@@ -166,6 +166,9 @@ struct Solver {
                 if ((int)(v - target) >= 0) break;
                 if (clock64() - t0 > kWaitLimit) {
                     s.failed = 1;
+                    // the host looks here too: the CTA that came last may pass, and
+                    // the first CTA finish the solve, without this one's rows
+                    *static_cast<volatile unsigned *>(a.barrier + 1) = 1;
                     break;
                 }
             }
@@ -442,7 +445,7 @@ cudaError_t launch_gmres_small(SmallGmresArgs a, double *work, int sm_count, cud
     a.xcur = a.w + a.n;
     cudaError_t e = cudaFuncSetAttribute(gmres_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)sizeof(Shared));
-    if (e == cudaSuccess) e = cudaMemsetAsync(a.barrier, 0, sizeof(unsigned), st);
+    if (e == cudaSuccess) e = cudaMemsetAsync(a.barrier, 0, 2 * sizeof(unsigned), st);
     if (e != cudaSuccess) return e;
     void *args[] = {&a};
     return cudaLaunchCooperativeKernel(reinterpret_cast<void *>(gmres_small_kernel), dim3(sm_count), dim3(kThreads), args,

@@ -353,7 +353,7 @@ struct SmallGmresArgs {
     double tol;
     const double *b;
     double *x;                // the initial guess, then the solution
-    unsigned *barrier;        // device word
+    unsigned *barrier;        // device: arrivals; then whether a CTA gave up waiting
     SmallGmresStat *stat;     // device
     // set by the launcher
     double *sums, *w, *xcur;
