@@ -275,7 +275,12 @@ rf_status rf_profile_matvec(rf_handle *h, int32_t reps, double *ms_per_product, 
  * GMRES otherwise) with events on the handle's stream; enable = 0 stops.
  * Either way *count, *total_ms and *bytes_per_product report the products
  * timed since the last reset, their summed device time and the bytes of A one
- * product streams.  Pointers may be NULL. */
+ * product streams.  Pointers may be NULL.
+ * A small FP64 system (n <= 8192, restart <= 16, no preconditioner) is otherwise
+ * solved by one kernel, whose products no event can bracket: with the timer on
+ * it takes the launched passes of larger systems, the same steps with sums in
+ * another order (results equal to rounding) at two to three times the solve's
+ * time, so that what is timed are those passes' products. */
 rf_status rf_gemv_timer(rf_handle *h, int32_t enable, int64_t *count, double *total_ms, double *bytes_per_product);
 
 /* Sizes. */

@@ -358,7 +358,9 @@ class Simulation:
 
     def gemv_timer(self, enable):
         """Start (True, counters reset) or stop live timing of the inner-solve
-        products; returns (products timed, their total ms, bytes of A per product)."""
+        products; returns (products timed, their total ms, bytes of A per product).
+        With the timer on, a small FP64 system (n <= 8192) leaves its single-kernel
+        solver for launched passes (rf_gemv_timer): equal to rounding, but slower."""
         cnt, ms, nbytes = ctypes.c_int64(), ctypes.c_double(), ctypes.c_double()
         L.check(L.lib().rf_gemv_timer(self._h, 1 if enable else 0, ctypes.byref(cnt), ctypes.byref(ms),
                                       ctypes.byref(nbytes)), self._h)
