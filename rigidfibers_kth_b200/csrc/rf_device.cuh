@@ -96,14 +96,18 @@ __device__ __forceinline__ double rsqrt_pos(double x) {
     const double e = fma(-x * y, y, 1.0);
     return fma(y * e, fma(0.375, e, 0.5), y);
 }
-// a / b from y = 1/b (within two units), and sqrt(x): one correction with the
-// exact remainder (Markstein 1990, as div_const), off by less than 2^-50 units
-// before its rounding: the correctly rounded value except where the quotient
-// or root lies that close to a rounding boundary.  The compiler's division and
-// square root branch to a path for subnormal and special operands, so that the
-// ten divisions of the closed forms run one after the other; these interleave,
-// and quotients of one denominator share its reciprocal.  A zero or infinite
-// operand gives NaN (the reference's formulas are singular there).
+// a / b from y = 1/b within u units (2^-53, relative; u is 2 for rcp_pos(b) and
+// below 13 for the products of reciprocals that the closed forms pass), and
+// sqrt(x): one correction with the remainder (Markstein 1990, as div_const).
+// The quotient to be corrected is within u + 1 units, the remainder formed to a
+// rounding of itself, so that the corrected sum is off by less than (u + 1)
+// (u + 2) 2^-53 units before its rounding, 2^-45 at the most: the correctly
+// rounded value except where the quotient or root lies that close to a rounding
+// boundary.  The compiler's division and square root branch to a path for
+// subnormal and special operands, so that the ten divisions of the closed forms
+// run one after the other; these interleave, and quotients of one denominator
+// share its reciprocal.  A zero or infinite operand gives NaN (the reference's
+// formulas are singular there).
 __device__ __forceinline__ double div_by(double a, double b, double y) {
     const double q = __dmul_rn(a, y);
     return __fma_rn(__fma_rn(-q, b, a), y, q);
