@@ -517,12 +517,16 @@ __global__ void __launch_bounds__(kTrsmThreads) lu_trsm_kernel(double *A, int64_
 
 // C -= A B on the FP64 tensor cores (mma.sync m8n8k4): A m x kLuNb, B kLuNb x
 // nc, C m x nc, all column-major with ld lda and 16-byte aligned starts.  A CTA
-// of four warps owns a 128 x 64 tile, a warp 64 x 32 of it in registers
-// (starting from -C, so that the result is -acc); operands in k-blocks of 16
-// through a ring of three stages (cp.async).  Two CTAs per SM: one's C traffic
-// (two passes over the trailing matrix per 128 columns) hides behind the
-// other's products.  Row strides of 4 mod 16 doubles keep the operand loads
-// free of bank conflicts.
+// of four warps owns a 128 x 64 tile, a warp 64 x 32 of it in registers;
+// operands in k-blocks of 16 through a ring of three stages (cp.async).  The
+// products are summed by themselves and C taken off behind the second half of
+// the k-blocks, a thread's rows in turn (on average 28 of 128 products are
+// added to sums that hold C).  Summed onto C from the start, every product was
+// rounded at C's size: error of a solution at n = 2500 2.8e-15, from zero with C
+// loaded at the end 0.8e-15 but 174 instead of 126 ms at n = 15000; this way
+// 1.5e-15 (LAPACK's 1.4e-15) and 122 ms, C's loads now behind the products.  Two
+// CTAs per SM: one's C traffic hides behind the other's products.  Row strides
+// of 4 mod 16 doubles keep the operand loads free of bank conflicts.
 constexpr int kGM = 128, kGN = 64, kGK = 16, kGStages = 3, kGThreads = 128;
 constexpr int kGLdA = kGM + 4, kGLdB = kGK + 4;
 constexpr size_t kGStage = sizeof(double) * (kGK * kGLdA + kGN * kGLdB);
@@ -544,23 +548,25 @@ __global__ void __launch_bounds__(kGThreads, 2) lu_gemm_kernel(const double *__r
     extern __shared__ __align__(16) double smem[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int64_t r0 = (int64_t)blockIdx.x * kGM, c0 = (int64_t)blockIdx.y * kGN;
+    // within the tile 32-bit offsets do (128 columns of less than 2^24 rows)
+    A += r0;
+    B += c0 * lda;
+    C += c0 * lda + r0;
+    const int ld = (int)lda, rows = (int)std::min<int64_t>(m - r0, kGM), cols = (int)std::min<int64_t>(nc - c0, kGN);
     auto stage_a = [&](int st) { return smem + st * (kGK * kGLdA + kGN * kGLdB); };
     auto stage_b = [&](int st) { return stage_a(st) + kGK * kGLdA; };
     auto load = [&](int kb) {
         double *sa = stage_a(kb % kGStages), *sb = stage_b(kb % kGStages);
-        const int64_t k0 = (int64_t)kb * kGK;
+        const int k0 = kb * kGK;
 #pragma unroll
         for (int t = 0; t < kGK * kGM / 2 / kGThreads; ++t) {
             const int e = t * kGThreads + tid, q = e / (kGM / 2), r = 2 * (e % (kGM / 2));
-            const int64_t left = m - r0 - r;
-            cp16(sa + q * kGLdA + r, A + (k0 + q) * lda + (left > 0 ? r0 + r : 0),
-                 left >= 2 ? 16 : left == 1 ? 8 : 0);
+            cp16(sa + q * kGLdA + r, A + (k0 + q) * ld + (r < rows ? r : 0), r + 1 < rows ? 16 : r < rows ? 8 : 0);
         }
 #pragma unroll
         for (int t = 0; t < kGN * kGK / 2 / kGThreads; ++t) {
             const int e = t * kGThreads + tid, c = e / (kGK / 2), q = 2 * (e % (kGK / 2));
-            const bool in = c0 + c < nc;
-            cp16(sb + c * kGLdB + q, B + (in ? c0 + c : 0) * lda + k0 + q, in ? 16 : 0);
+            cp16(sb + c * kGLdB + q, B + (c < cols ? c : 0) * ld + k0 + q, c < cols ? 16 : 0);
         }
     };
     constexpr int KB = kLuNb / kGK;
@@ -573,26 +579,20 @@ __global__ void __launch_bounds__(kGThreads, 2) lu_gemm_kernel(const double *__r
     const int g = lane >> 2, q4 = lane & 3;
     double acc[8][4][2];
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
+    for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int64_t c = c0 + wc + 8 * j + 2 * q4 + h;
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const int64_t r = r0 + wr + 8 * i + g;
-                acc[i][j][h] = r < m && c < nc ? -C[c * lda + r] : 0.0;
-            }
-        }
-#pragma unroll 1
-    for (int kb = 0; kb < KB; ++kb) {
+        for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+    auto arrive = [&](int kb) {
         cp_wait<kGStages - 2>();
         __syncthreads();  // stage kb has arrived for every thread, stage kb - 1 has been read
         if (kb + kGStages - 1 < KB) load(kb + kGStages - 1);
         cp_commit();
+    };
+    auto products = [&](int kb, int s0, int s1) {
         const double *sa = stage_a(kb % kGStages) + q4 * kGLdA + wr + g;
         const double *sb = stage_b(kb % kGStages) + (wc + g) * kGLdB + q4;
 #pragma unroll
-        for (int s = 0; s < kGK; s += 4) {
+        for (int s = s0; s < s1; s += 4) {
             double a[8], b[4];
 #pragma unroll
             for (int i = 0; i < 8; ++i) a[i] = sa[s * kGLdA + 8 * i];
@@ -604,16 +604,40 @@ __global__ void __launch_bounds__(kGThreads, 2) lu_gemm_kernel(const double *__r
                 for (int j = 0; j < 4; ++j)
                     dmma_8x8x4(acc[i][j][0], acc[i][j][1], a[i], b[j], acc[i][j][0], acc[i][j][1]);
         }
+    };
+#pragma unroll 1
+    for (int kb = 0; kb < KB / 2; ++kb) {
+        arrive(kb);
+        products(kb, 0, kGK);
+    }
+    // C comes in behind the second half, the values of one of a thread's rows at a
+    // time (addresses clamped to the tile, not predicated: branches here took 57
+    // doubles of local memory)
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int kb = KB / 2 + i / 2;
+        double old[4][2];
+        const int r = min(wr + 8 * i + g, rows - 1);  // beyond the tile: never stored
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) old[j][h] = C[min(wc + 8 * j + 2 * q4 + h, cols - 1) * ld + r];
+        if (i % 2 == 0) arrive(kb);
+        products(kb, i % 2 * (kGK / 2), (i % 2 + 1) * (kGK / 2));
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) acc[i][j][h] -= old[j][h];
     }
 #pragma unroll
     for (int j = 0; j < 4; ++j)
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-            const int64_t c = c0 + wc + 8 * j + 2 * q4 + h;
+            const int c = wc + 8 * j + 2 * q4 + h;
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
-                const int64_t r = r0 + wr + 8 * i + g;
-                if (r < m && c < nc) C[c * lda + r] = -acc[i][j][h];
+                const int r = wr + 8 * i + g;
+                if (r < rows && c < cols) C[c * ld + r] = -acc[i][j][h];
             }
         }
 }
