@@ -21,16 +21,16 @@
 // them again.  Info as LAPACK: the first zero pivot (1-based), 0 when there
 // is none.
 //
-// What bounds it (n = 15000): the trailing updates, 83 of 126 ms = 27 of 37
+// What bounds it (n = 15000): the trailing updates, 78 of 122 ms = 29 of 37
 // TFLOP/s (128-column panels: the 64-column panels of a cuBLAS GEMM before
 // passed twice as often over the trailing matrix, 107 ms), then the panels, 31
 // ms: 1.4 us a column, three quarters of it latencies of the pivot search, the
 // exchange and the cluster barrier.  Before, a panel went through memory eight
 // columns at a time (92 ms, and 36 ms of rank-8 updates), the triangles ran one
 // thread per column through global memory and the forward substitution panel
-// by panel.  Factor and solve: n = 15000 234 -> 126 ms, n = 4500 37 -> 13 ms,
-// n = 1500 10.8 -> 3.5 ms, n = 300 2.0 -> 0.7 ms; rf_dgesv n = 3001 with its
-// copies 33 -> 17 ms.
+// by panel.  Factor and solve: n = 15000 234 -> 122 ms, n = 4500 37 -> 13 ms,
+// n = 1500 10.7 -> 3.4 ms, n = 300 2.0 -> 0.7 ms; rf_dgesv n = 3001 with its
+// copies 34 -> 17 ms.
 #include <cooperative_groups.h>
 
 #include <algorithm>
@@ -648,8 +648,8 @@ __global__ void __launch_bounds__(kGThreads, 2) lu_gemm_kernel(const double *__r
 // warps.  Quotients come from each lane's reciprocal; a block in which a pivot,
 // an operand or a quotient is zero, not finite or near the ends of the range is
 // solved again with divisions (a subnormal or huge pivot has no usable
-// reciprocal; overflow and underflow need the division's own rounding).  The
-// choice per quotient instead cost 50 ns a row, 0.8 of 127 ms at n = 15000.
+// reciprocal; overflow and underflow need the division's own rounding).  A
+// choice per quotient stood in the serial chain: 20.5 instead of 15.1 us a block.
 constexpr int kBackThreads = 512;
 constexpr int kBackLd = kLuNb + 1;
 __global__ void __launch_bounds__(kBackThreads) lu_back_diag_kernel(const double *__restrict__ A, int64_t lda,
@@ -670,22 +670,20 @@ __global__ void __launch_bounds__(kBackThreads) lu_back_diag_kernel(const double
         if (tid < 32) {
             const double x0 = lane < bn ? s_x[b + lane] : 0.0, d = lane < bn ? s_u[(b + lane) * kBackLd + b + lane] : 1.0;
             const double rd = copysign(rcp_pos(fabs(d)), d);
+            double num;  // what the lane's quotient was formed from
             auto solve = [&](auto quotient) {
-                double xi = x0;
+                double xi = num = x0;
                 for (int p = bn - 1; p >= 0; --p) {
                     const double u = lane < p ? s_u[(b + p) * kBackLd + b + lane] : 0.0;
-                    if (lane == p) xi = quotient(xi);
+                    const double q = quotient(xi);  // every lane's: no branch
+                    if (lane == p) num = xi, xi = q;
                     const double xp = __shfl_sync(0xffffffffu, xi, p);
                     if (lane < p) xi = fma(-u, xp, xi);
                 }
                 return xi;
             };
-            bool ok = mid_range(d);
-            double xi = solve([&](double v) {
-                const double q = div_by(v, d, rd);
-                ok = ok && mid_range(v) && mid_range(q);
-                return q;
-            });
+            double xi = solve([&](double v) { return div_by(v, d, rd); });
+            const bool ok = mid_range(d) && mid_range(num) && mid_range(xi);
             if (__any_sync(0xffffffffu, !ok && lane < bn)) xi = solve([&](double v) { return v / d; });
             if (lane < bn) s_x[b + lane] = xi;
         }
