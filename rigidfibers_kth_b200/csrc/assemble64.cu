@@ -30,7 +30,7 @@
 // M = 1000 with N = 2 2.0 -> 1.2 ms, M = 1000 with panels 3.8 -> 2.0 ms.
 //
 // What bounds it: the FP64 pipe (M = 1000 cloud: 54 % busy and the FP64
-// tensor cores, which share it, 9.5 %) with 14 resident warps per SM (124
+// tensor cores, which share it, 9.5 %) with 14 resident warps per SM (122
 // registers, 54 KB of shared memory per CTA: four CTAs); the stalls that are
 // left are fixed latencies (2.2 warps per issue) and the pipe itself (1.6).
 // Unrolling the recursion and P3 over its lanes' items made the code exceed
